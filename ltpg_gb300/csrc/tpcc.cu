@@ -528,6 +528,7 @@ __global__ void __launch_bounds__(PBS) tpcc_writeback_plain(const ltpg_tpcc_txn 
     __shared__ TileHdr h;
     __shared__ uint8_t fl[PT];
     const uint32_t t0 = blockIdx.x * PT, nt = min(PT, B - t0);
+    TxnCounts cnt;
     if (threadIdx.x < PT) {
         const uint32_t f = threadIdx.x < nt ? flags[t0 + threadIdx.x] : 0u;
         fl[threadIdx.x] = (uint8_t)f;
@@ -537,13 +538,10 @@ __global__ void __launch_bounds__(PBS) tpcc_writeback_plain(const ltpg_tpcc_txn 
         const unsigned bwaw = __ballot_sync(FULL, (f & LTPG_FLAG_WAW) != 0u);
         if ((threadIdx.x & 31) == 0 && threadIdx.x < nt) {
             bitmap[(t0 + threadIdx.x) >> 5] = bal;
-            if (bal) {
-                red_add_u64(&st->commits, __popc(bal));
-                red_add_u64(&ctl->total_commits, __popc(bal));
-            }
-            if (braw) red_add_u64(&st->raw, __popc(braw));
-            if (bwar) red_add_u64(&st->war, __popc(bwar));
-            if (bwaw) red_add_u64(&st->waw, __popc(bwaw));
+            cnt.com = __popc(bal);
+            cnt.raw = __popc(braw);
+            cnt.war = __popc(bwar);
+            cnt.waw = __popc(bwaw);
         }
     }
     __syncthreads();
@@ -554,7 +552,8 @@ __global__ void __launch_bounds__(PBS) tpcc_writeback_plain(const ltpg_tpcc_txn 
         const uint32_t i = tile_owner(h, nt, e), q = e - h.off[i];
         tpcc_apply_write<true>(db, h.x[i], q, lines, txn_base + t0 + i, nullptr, nullptr, results[t0 + i]);
     }
-    finish_batch(ctl);
+    add_counters(st, ctl, cnt);
+    finish_batch<false>(ctl);
 }
 
 cudaError_t tpcc_phase(ltpg_ctx *c, Slot &s, int phase) {
@@ -760,14 +759,14 @@ __device__ __forceinline__ void tpcc_exec_tiles(const TpccTunedArgs &a, TileHdrN
 
 // hot: 11 W int64 sums in shared memory (W <= HOT_SMEM_MAX_W), or null.
 template <uint32_t P>
-__device__ __forceinline__ void tpcc_checkwb_tiles(const TpccTunedArgs &a, TileHdrN<P> &h, uint32_t epoch,
-                                                   long long *hot) {
+__device__ __forceinline__ TxnCounts tpcc_checkwb_tiles(const TpccTunedArgs &a, TileHdrN<P> &h, uint32_t epoch,
+                                                        long long *hot) {
     const uint32_t n_lines = (uint32_t)a.hdr[0];
     const uint64_t txn_base = a.hdr[1];
     __shared__ uint32_t fl[P];
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t n_tiles = (a.B + P - 1) / P;
-    unsigned long long c_com = 0, c_raw = 0, c_war = 0, c_waw = 0;
+    TxnCounts cnt;
     for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
         const uint32_t t0 = tile * P, nt = min(P, a.B - t0);
         if (threadIdx.x < P) fl[threadIdx.x] = 0u;
@@ -813,10 +812,10 @@ __device__ __forceinline__ void tpcc_checkwb_tiles(const TpccTunedArgs &a, TileH
             const unsigned bwaw = __ballot_sync(FULL, (f & LTPG_FLAG_WAW) != 0u);
             if (lane == 0 && threadIdx.x < nt) {
                 a.bitmap[(t0 + threadIdx.x) >> 5] = bal;
-                c_com += __popc(bal);
-                c_raw += __popc(braw);
-                c_war += __popc(bwar);
-                c_waw += __popc(bwaw);
+                cnt.com += __popc(bal);
+                cnt.raw += __popc(braw);
+                cnt.war += __popc(bwar);
+                cnt.waw += __popc(bwaw);
             }
         }
         __syncthreads();
@@ -843,23 +842,15 @@ __device__ __forceinline__ void tpcc_checkwb_tiles(const TpccTunedArgs &a, TileH
         }
         __syncthreads();
     }
-    if (lane == 0) {
-        if (c_com) {
-            red_add_u64(&a.st->commits, c_com);
-            red_add_u64(&a.ctl->total_commits, c_com);
-        }
-        if (c_raw) red_add_u64(&a.st->raw, c_raw);
-        if (c_war) red_add_u64(&a.st->war, c_war);
-        if (c_waw) red_add_u64(&a.st->waw, c_waw);
-    }
+    return cnt;
 }
 
 __device__ __forceinline__ void hot_init(long long *hot, uint32_t n) {
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) hot[i] = 0;
     __syncthreads();
 }
+// After the last tile's barrier, or hot_init's.
 __device__ __forceinline__ void hot_flush(const TpccDev &db, const long long *hot) {
-    __syncthreads();
     for (uint32_t i = threadIdx.x; i < 11u * db.W; i += blockDim.x) {
         const long long v = hot[i];
         if (!v) continue;
@@ -880,9 +871,10 @@ __global__ void __launch_bounds__(2 * P) tpcc_checkwb_tuned(TpccTunedArgs a) {
     extern __shared__ __align__(16) long long hot_dyn[];
     long long *hot = a.db.W <= HOT_SMEM_MAX_W ? hot_dyn : nullptr;
     if (hot) hot_init(hot, 11u * a.db.W);
-    tpcc_checkwb_tiles<P>(a, h, a.ctl->epoch, hot);
+    const TxnCounts cnt = tpcc_checkwb_tiles<P>(a, h, a.ctl->epoch, hot);
     if (hot) hot_flush(a.db, hot);
-    finish_batch(a.ctl);
+    add_counters(a.st, a.ctl, cnt);
+    finish_batch<false>(a.ctl);
 }
 
 // One cooperative kernel per batch: execute+register, a bounded grid barrier,
@@ -901,9 +893,11 @@ __global__ void __launch_bounds__(2 * P) tpcc_persistent(TpccTunedArgs a) {
     const uint32_t epoch = a.ctl->epoch;
     if (hot) hot_init(hot, 11u * a.db.W);
     tpcc_exec_tiles<P>(a, h, slot_tag(epoch));
-    if (grid_barrier(a.ctl)) tpcc_checkwb_tiles<P>(a, h, epoch, hot);
+    TxnCounts cnt;
+    if (grid_barrier(a.ctl)) cnt = tpcc_checkwb_tiles<P>(a, h, epoch, hot);
     if (hot) hot_flush(a.db, hot);
-    finish_batch(a.ctl);
+    add_counters(a.st, a.ctl, cnt);
+    finish_batch<false>(a.ctl);
 }
 
 template <uint32_t P>

@@ -120,16 +120,7 @@ __global__ void __launch_bounds__(256) ycsb_writeback_plain(const uint8_t *__res
     const unsigned braw = __ballot_sync(FULL, (f & LTPG_FLAG_RAW) != 0u);
     const unsigned bwar = __ballot_sync(FULL, (f & LTPG_FLAG_WAR) != 0u);
     const unsigned bwaw = __ballot_sync(FULL, (f & LTPG_FLAG_WAW) != 0u);
-    if (lane == 0 && t < B) {
-        bitmap[t >> 5] = bal;
-        if (bal) {
-            red_add_u64(&st->commits, __popc(bal));
-            red_add_u64(&ctl->total_commits, __popc(bal));
-        }
-        if (braw) red_add_u64(&st->raw, __popc(braw));
-        if (bwar) red_add_u64(&st->war, __popc(bwar));
-        if (bwaw) red_add_u64(&st->waw, __popc(bwaw));
-    }
+    if (lane == 0 && t < B) bitmap[t >> 5] = bal;
     if (com && val_off[t + 1] != val_off[t]) {
         // value indices stay below the batch's value count and the buffer's
         // capacity: offsets that disagree with the op words (a malformed
@@ -149,7 +140,9 @@ __global__ void __launch_bounds__(256) ycsb_writeback_plain(const uint8_t *__res
             ++v;
         }
     }
-    finish_batch(ctl);
+    add_counters(st, ctl, TxnCounts{(uint32_t)__popc(bal), (uint32_t)__popc(braw), (uint32_t)__popc(bwar),
+                                    (uint32_t)__popc(bwaw)});
+    finish_batch<false>(ctl);
 }
 
 // ---- value offsets made on the device -------------------------------------------

@@ -576,7 +576,7 @@ __device__ __forceinline__ void checkwb_tiles(const YcsbTunedArgs &a, uint32_t *
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t nvec_tile = a.tile * a.stride / 4;
     const uint32_t n_tiles = (a.B + a.tile - 1) / a.tile;
-    unsigned long long c_com = 0, c_raw = 0, c_war = 0, c_waw = 0;
+    TxnCounts cnt;
     for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
         const uint32_t t0 = tile * a.tile;
         const uint32_t nt = min(a.tile, a.B - t0);
@@ -624,10 +624,10 @@ __device__ __forceinline__ void checkwb_tiles(const YcsbTunedArgs &a, uint32_t *
             const unsigned bwaw = __ballot_sync(FULL, (f & LTPG_FLAG_WAW) != 0u);
             if (lane == 0 && i < nt) {
                 a.bitmap[(t0 + i) >> 5] = bal;
-                c_com += __popc(bal);
-                c_raw += __popc(braw);
-                c_war += __popc(bwar);
-                c_waw += __popc(bwaw);
+                cnt.com += __popc(bal);
+                cnt.raw += __popc(braw);
+                cnt.war += __popc(bwar);
+                cnt.waw += __popc(bwaw);
             }
         }
         __syncthreads();
@@ -641,15 +641,7 @@ __device__ __forceinline__ void checkwb_tiles(const YcsbTunedArgs &a, uint32_t *
         }
         __syncthreads();
     }
-    if (lane == 0) {
-        if (c_com) {
-            red_add_u64(&a.st->commits, c_com);
-            red_add_u64(&a.ctl->total_commits, c_com);
-        }
-        if (c_raw) red_add_u64(&a.st->raw, c_raw);
-        if (c_war) red_add_u64(&a.st->war, c_war);
-        if (c_waw) red_add_u64(&a.st->waw, c_waw);
-    }
+    add_counters(a.st, a.ctl, cnt);
 }
 
 // ---- fast execute+register: transactions of 2^m words, no block barriers -----
@@ -1011,7 +1003,7 @@ __global__ void __launch_bounds__(512) ycsb_checkwb_tuned(YcsbTunedArgs a) {
     extern __shared__ __align__(16) char smem[];
     const SmemPtrs p = carve(smem, a.tile);
     checkwb_tiles<kLate>(a, p.fl, a.ctl->epoch);
-    if (!kLate) finish_batch(a.ctl);
+    if (!kLate) finish_batch<false>(a.ctl);
 }
 
 // Write-back after late reads: one thread per transaction; a committed one
@@ -1021,10 +1013,10 @@ __global__ void __launch_bounds__(512) ycsb_checkwb_tuned(YcsbTunedArgs a) {
 // one bitmap word) and the counters.  kStore = false: the decision only (the
 // update-list write-back stores from the list).
 template <bool kDecide, bool kCoh, bool kStore = true>
-__device__ __forceinline__ void writeback_late_loop(const YcsbTunedArgs &a) {
+__device__ __forceinline__ TxnCounts writeback_late_loop(const YcsbTunedArgs &a) {
     const uint32_t step = gridDim.x * blockDim.x;
     const uint32_t lane = threadIdx.x & 31;
-    unsigned long long c_com = 0, c_raw = 0, c_war = 0, c_waw = 0;
+    TxnCounts cnt;
     for (uint32_t base = blockIdx.x * blockDim.x; base < a.B; base += step) {
         const uint32_t t = base + threadIdx.x;
         const bool act = t < a.B;
@@ -1039,25 +1031,17 @@ __device__ __forceinline__ void writeback_late_loop(const YcsbTunedArgs &a) {
             const unsigned bww = __ballot_sync(FULL, (f & LTPG_FLAG_WAW) != 0u);
             if (lane == 0u && act) {
                 a.bitmap[t >> 5] = bc;
-                c_com += __popc(bc);
-                c_raw += __popc(br);
-                c_war += __popc(bwr);
-                c_waw += __popc(bww);
+                cnt.com += __popc(bc);
+                cnt.raw += __popc(br);
+                cnt.war += __popc(bwr);
+                cnt.waw += __popc(bww);
             }
         } else {
             com = (f & LTPG_FLAG_COMMIT) != 0u;
         }
         if (kStore && com) write_txn_updates(a, t);
     }
-    if (kDecide && lane == 0u) {
-        if (c_com) {
-            red_add_u64(&a.st->commits, c_com);
-            red_add_u64(&a.ctl->total_commits, c_com);
-        }
-        if (c_raw) red_add_u64(&a.st->raw, c_raw);
-        if (c_war) red_add_u64(&a.st->war, c_war);
-        if (c_waw) red_add_u64(&a.st->waw, c_waw);
-    }
+    return cnt;
 }
 
 // Late reads 2: the check kernel made the decisions; this one stores.
@@ -1077,7 +1061,7 @@ __global__ void __launch_bounds__(BS) ycsb_writeback_late(YcsbTunedArgs a) {
 // loop adds COMMIT to it decides the same.
 template <bool kCoh>
 __device__ __forceinline__ void writeback_list(const YcsbTunedArgs &a) {
-    writeback_late_loop<true, kCoh, false>(a);
+    const TxnCounts cnt = writeback_late_loop<true, kCoh, false>(a);
     // a batch whose registration reported an error (a key past the table, or
     // offsets that disagree with the op words, which leave list positions
     // unwritten) stores nothing
@@ -1096,11 +1080,12 @@ __device__ __forceinline__ void writeback_list(const YcsbTunedArgs &a) {
         }
         if (last && u < a.vals_cap) a.rows[(uint64_t)key * LTPG_YCSB_FIELDS + fld] = __ldg(a.vals + u);
     }
+    add_counters(a.st, a.ctl, cnt);
 }
 template <int BS>
 __global__ void __launch_bounds__(BS) ycsb_writeback_list(YcsbTunedArgs a) {
     writeback_list<false>(a);
-    finish_batch(a.ctl);
+    finish_batch<false>(a.ctl);
 }
 
 // One cooperative kernel per batch: execute+register, grid barrier, check +
@@ -1126,7 +1111,8 @@ __device__ __forceinline__ void ycsb_persistent_body(const YcsbTunedArgs &a) {
         if (ok) late_read_loop<true>(a);
         ok = ok && grid_barrier(a.ctl);
         if (ok) writeback_list<true>(a);
-        finish_batch(a.ctl);
+        if (ok) finish_batch<false>(a.ctl);
+        else finish_batch(a.ctl);
         return;
     }
     if (kStage) {
@@ -1158,7 +1144,8 @@ __device__ __forceinline__ void ycsb_persistent_body(const YcsbTunedArgs &a) {
         ok = ok && grid_barrier(a.ctl);
         if (ok) writeback_late_loop<false, true>(a);
     }
-    finish_batch(a.ctl);
+    if (!kLate && ok) finish_batch<false>(a.ctl);
+    else finish_batch(a.ctl);
 }
 template <bool kStage, bool kLate>
 __global__ void __launch_bounds__(512) ycsb_persistent(YcsbTunedArgs a) { ycsb_persistent_body<kStage, kLate>(a); }
