@@ -202,65 +202,126 @@ __device__ __forceinline__ void write_txn_updates(const YcsbTunedArgs &a, uint32
 // its contiguous rows.  results[t] = sum over reads of xor(row) * (2j + 1), as
 // at execute; 0 for an aborted transaction.  No row is written before the
 // next kernel, so every read sees the batch-start image.
-// Per-warp shared scratch of the late reads: the keys of the warp's point
-// reads by rank, and the xor of each one's row.
-struct LateScratch {
+// Row gather of a warp: the rows of up to 32 keys, five lanes to a row (one
+// 16-byte chunk each, six rows per round on lanes 0..29), so a row costs one or
+// two cache-line requests.  `need` (a ballot) names the lanes that want a row;
+// a lane's rank among them is its row's number.  Per-warp shared scratch: the
+// keys by rank, and each chunk's xor at 5 * rank + chunk = 30 * round + lane,
+// from where a row's owner folds its five (stride 40 bytes: no bank conflict).
+// Folding through shared memory takes one store per round and five loads per
+// warp, where shuffles took six per round: the late-read kernel was issue-bound
+// (2^20 x 16 at theta 0.99: 190 -> 172 us, 100 G random sectors/s of DRAM; a
+// 10,000 x 10 persistent batch with reads at execute 27.6 -> 25.2 us).
+// Three rounds (18 rows) are folded at a time, which keeps the scratch of a
+// 256-thread block below 7 KB (what shared memory takes, L1 loses).
+struct RowScratch {
     uint32_t key[32];
-    unsigned long long x[32];
+    unsigned long long part[90];
 };
 
-// This warp's scratch; one array per kernel, whichever late-read loops it runs.
-__device__ __forceinline__ LateScratch *late_scratch() {
-    __shared__ LateScratch scratch[16];  // blocks of up to 512 threads
+// This warp's scratch; one array per kernel, whichever row-reading loops it
+// runs, sized by the kernel's launch bounds.
+template <int BS>
+__device__ __forceinline__ RowScratch *row_scratch() {
+    __shared__ RowScratch scratch[BS / 32];
     return scratch + (threadIdx.x >> 5);
+}
+
+// Puts the keys in place and issues every chunk load of the gather.
+__device__ __forceinline__ void rows_issue(const uint64_t *rows, RowScratch *ws, uint32_t key, unsigned need,
+                                           ulonglong2 *ch) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t n5 = lane < 30u ? 5u * __popc(need) : 0u;
+    if ((need >> lane) & 1u) ws->key[__popc(need & ((1u << lane) - 1u))] = key;
+    __syncwarp();
+    const char *base = reinterpret_cast<const char *>(rows) + 16u * (lane % 5u);
+    const uint32_t grp = lane / 5u;
+#pragma unroll
+    for (uint32_t r = 0; r < 6; ++r) {
+        ch[r] = make_ulonglong2(0ull, 0ull);
+        if (30u * r + lane < n5)
+            ch[r] = ld_nc16_issue(base + (uint64_t)ws->key[6u * r + grp] * (8u * LTPG_YCSB_FIELDS));
+    }
+}
+
+// The xor of the row of each lane in `need` (0 for the other lanes).
+__device__ __forceinline__ unsigned long long rows_fold(RowScratch *ws, unsigned need, const ulonglong2 *ch) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t n = __popc(need), n5 = lane < 30u ? 5u * n : 0u;
+    const uint32_t rank = __popc(need & ((1u << lane) - 1u));
+    unsigned long long x = 0;
+#pragma unroll
+    for (uint32_t h = 0; h < 2; ++h) {
+        if (h) {
+            if (n <= 18u) break;  // warp-uniform
+            __syncwarp();
+        }
+#pragma unroll
+        for (uint32_t r = 0; r < 3; ++r)
+            if (90u * h + 30u * r + lane < n5) ws->part[30u * r + lane] = ch[3u * h + r].x ^ ch[3u * h + r].y;
+        __syncwarp();
+        if (((need >> lane) & 1u) && rank - 18u * h < 18u) {
+            const unsigned long long *p = ws->part + 5u * (rank - 18u * h);
+            x = p[0] ^ p[1] ^ p[2] ^ p[3] ^ p[4];
+        }
+    }
+    // the next gather writes `part` after its own barrier, and `key` before it:
+    // every key was read before this fold's first barrier
+    return x;
+}
+
+// The same gather with no shared memory: round r searches the ballot for the
+// (6r + g)-th row of group g, and shuffles fold the chunks and hand the row's
+// xor to its owner.  The staged kernels use it: their table takes 48 KB a
+// block, and its shared-memory atomics queue behind the other form's stores and
+// loads (2^18 x 16 at theta 0.99, 42 % of the ops staged: 228 us against 304).
+__device__ __forceinline__ void rows_issue_shfl(const uint64_t *rows, uint32_t key, unsigned need, ulonglong2 *ch) {
+    const uint32_t lane = threadIdx.x & 31, grp = lane / 5u, n = __popc(need);
+#pragma unroll
+    for (uint32_t r = 0; r < 6; ++r) {
+        const uint32_t idx = r * 6u + grp;
+        const bool go = grp < 6u && idx < n;
+        const uint32_t src = go ? __fns(need, 0, (int)idx + 1) : 0u;
+        const uint32_t k_src = __shfl_sync(FULL, key, src & 31u);
+        ch[r] = go ? ld_nc16_issue(reinterpret_cast<const char *>(rows + (uint64_t)k_src * LTPG_YCSB_FIELDS) +
+                                   16u * (lane % 5u))
+                   : make_ulonglong2(0ull, 0ull);
+    }
+}
+__device__ __forceinline__ unsigned long long rows_fold_shfl(unsigned need, const ulonglong2 *ch) {
+    const uint32_t lane = threadIdx.x & 31, n = __popc(need), rank = __popc(need & ((1u << lane) - 1u));
+    unsigned long long x = 0;
+#pragma unroll
+    for (uint32_t r = 0; r < 6; ++r) {
+        if (r * 6u >= n) break;  // warp-uniform
+        // lane 5g: chunks 0 and 1, then 0..3, then chunk 4
+        const unsigned long long c0 = ch[r].x ^ ch[r].y;
+        unsigned long long c = c0 ^ __shfl_down_sync(FULL, c0, 1);
+        c ^= __shfl_down_sync(FULL, c, 2);
+        const unsigned long long rowx = c ^ __shfl_down_sync(FULL, c0, 4);
+        const unsigned long long got = __shfl_sync(FULL, rowx, ((rank - r * 6u) * 5u) & 31u);
+        if (((need >> lane) & 1u) && rank - r * 6u < 6u) x = got;
+    }
+    return x;
 }
 
 // One step of the lanes of a warp (all 32 call it): lane j of transaction t
 // (own: the lane holds an op slot of a transaction; com: t committed).
-__device__ __forceinline__ void late_read_step(const YcsbTunedArgs &a, LateScratch *ws, uint32_t t, uint32_t j,
+__device__ __forceinline__ void late_read_step(const YcsbTunedArgs &a, RowScratch *ws, uint32_t t, uint32_t j,
                                                bool own, bool com) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t lpt = a.lpt;
-    const uint32_t grp = lane / 5, chunk = lane % 5;
     {
         const uint32_t w = com && j < a.stride ? __ldg(a.ops + (uint64_t)t * a.stride + j) : LTPG_YCSB_OP_PAD;
         const uint32_t key = ycsb_key(w);
         const bool rd = !ycsb_is_pad(w) && !ycsb_is_update(w) && key < a.n;
         const bool scan = rd && ycsb_span(w) != 0u;
         const unsigned need = __ballot_sync(FULL, rd && !scan);
-        const uint32_t n_need = __popc(need);
         unsigned long long x = 0;
-        if (n_need) {  // warp-uniform
-            // round r: lane group g (five lanes, one 16-byte chunk each) reads
-            // the row of the (6r + g)-th point read; its first lane folds the
-            // chunks and leaves the row's xor under that rank
-            const uint32_t my_rank = __popc(need & ((1u << lane) - 1u));
-            const bool mine = (need >> lane) & 1u;
-            if (mine) ws->key[my_rank] = key;
-            __syncwarp();
+        if (need) {  // warp-uniform
             ulonglong2 ch[6];
-#pragma unroll
-            for (int r = 0; r < 6; ++r) {
-                const uint32_t idx = (uint32_t)r * 6u + grp;
-                const bool go = grp < 6 && idx < n_need;
-                const uint32_t k_src = go ? ws->key[idx] : 0u;
-                ch[r] = go ? ld_nc16_issue(reinterpret_cast<const char *>(a.rows + (uint64_t)k_src * LTPG_YCSB_FIELDS) +
-                                           16u * chunk)
-                           : make_ulonglong2(0ull, 0ull);
-            }
-#pragma unroll
-            for (int r = 0; r < 6; ++r) {
-                if ((uint32_t)r * 6u >= n_need) break;  // warp-uniform
-                const unsigned long long c0 = ch[r].x ^ ch[r].y;
-                unsigned long long c = c0 ^ __shfl_down_sync(FULL, c0, 1);
-                c ^= __shfl_down_sync(FULL, c, 2);
-                const unsigned long long rowx = c ^ __shfl_down_sync(FULL, c0, 4);
-                const uint32_t idx = (uint32_t)r * 6u + grp;
-                if (chunk == 0u && grp < 6 && idx < n_need) ws->x[idx] = rowx;
-            }
-            __syncwarp();
-            if (mine) x = ws->x[my_rank];
-            __syncwarp();  // the next step reuses the scratch
+            rows_issue(a.rows, ws, key, need, ch);
+            x = rows_fold(ws, need, ch);
         }
         const uint32_t last = scan ? (uint32_t)scan_last(w, a.n) : 0u;
         for (unsigned m = __ballot_sync(FULL, scan); m; m &= m - 1u) {
@@ -282,9 +343,8 @@ __device__ __forceinline__ void late_read_step(const YcsbTunedArgs &a, LateScrat
     }
 }
 
-__device__ __forceinline__ void late_read_tile(const YcsbTunedArgs &a, const uint32_t *fl, uint32_t t0,
+__device__ __forceinline__ void late_read_tile(const YcsbTunedArgs &a, RowScratch *ws, const uint32_t *fl, uint32_t t0,
                                                uint32_t nt) {
-    LateScratch *ws = late_scratch();
     const uint32_t lsh = (uint32_t)__ffs(a.lpt) - 1u;
     const uint32_t nl = a.tile << lsh;
     for (uint32_t base = 0; base < nl; base += blockDim.x) {
@@ -298,8 +358,7 @@ __device__ __forceinline__ void late_read_tile(const YcsbTunedArgs &a, const uin
 // Late reads as a kernel of their own (late_reads = 2), after the check: the
 // lanes of the whole batch, lpt per transaction, commit flags from global memory.
 template <bool kCoh>
-__device__ __forceinline__ void late_read_loop(const YcsbTunedArgs &a) {
-    LateScratch *ws = late_scratch();
+__device__ __forceinline__ void late_read_loop(const YcsbTunedArgs &a, RowScratch *ws) {
     const uint32_t lsh = (uint32_t)__ffs(a.lpt) - 1u;
     const uint64_t nw = (uint64_t)a.B << lsh;
     const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
@@ -320,7 +379,9 @@ __device__ __forceinline__ void late_read_loop(const YcsbTunedArgs &a) {
 // read kernel takes 58 registers under 512-thread bounds against 40 under
 // 256, and loses a third of its resident warps).
 template <int BS>
-__global__ void __launch_bounds__(BS) ycsb_read_late(YcsbTunedArgs a) { late_read_loop<false>(a); }
+__global__ void __launch_bounds__(BS) ycsb_read_late(YcsbTunedArgs a) {
+    late_read_loop<false>(a, row_scratch<BS>());
+}
 
 // ---- write-first registration (late_reads = 3) ---------------------------------
 // The same RAW / WAR / WAW outcome with at most one random slot access per op
@@ -351,14 +412,15 @@ __device__ __forceinline__ ulonglong2 ld_slot_ca(const RegSlot *p) {
 // Also zeroes the flag bytes, which (2) and (3) OR the conflict bits into.
 template <bool kCoh>
 __device__ __forceinline__ void wf_register_writes(const YcsbTunedArgs &a, uint64_t tag) {
-    const uint64_t nvec = (uint64_t)a.B * a.stride / 4u;
-    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ((uint64_t)a.B + 3) / 4; i += step)
+    // at most 2^26 transactions of 8 vectors: 32-bit indices (and divisions)
+    const uint32_t vpt = a.stride / 4u, nvec = a.B * vpt;
+    const uint32_t step = gridDim.x * blockDim.x;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (a.B + 3u) / 4u; i += step)
         reinterpret_cast<unsigned *>(a.flags)[i] = 0u;
     const uint4 *vp = reinterpret_cast<const uint4 *>(a.ops);
-    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < nvec; v += step) {
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nvec; v += step) {
         const uint4 w4 = ld_nc_u4(vp + v);
-        const uint32_t t = (uint32_t)(v * 4u / a.stride);
+        const uint32_t t = v / vpt;
         const uint32_t words[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -382,18 +444,40 @@ __device__ __forceinline__ void wf_register_writes(const YcsbTunedArgs &a, uint6
     }
 }
 
-// One key of a read: RAW against the final write word, registration when the
-// key has a writer.  Returns the RAW bit.  A key outside the writer bitmap has
-// no writer in the batch: no RAW, nothing to register, and no slot load (the
-// bitmap, 1/128 of the slot table, stays in L2).
+// One key of a read that has a writer: RAW against the final write word, and
+// the read's registration.  Returns the RAW bit.
 template <bool kCoh>
-__device__ __forceinline__ bool wf_read_key(const YcsbTunedArgs &a, uint64_t key, uint32_t t, uint32_t epoch,
-                                            unsigned long long mine) {
-    if (!((ld_wbits<kCoh>(a.wbits + (key >> 5)) >> (key & 31u)) & 1u)) return false;
-    const ulonglong2 s = kCoh ? ld_gpu_slot(a.reg + key) : ld_slot_ca(a.reg + key);
+__device__ __forceinline__ bool wf_read_key(const YcsbTunedArgs &a, uint32_t key, uint32_t t,
+                                            uint32_t epoch, const ulonglong2 &s) {
+    const unsigned long long mine = slot_tag(epoch) | t;
     const uint32_t wmin = slot_min(s.y, epoch);
     if (wmin != 0xFFFFFFFFu && s.x > mine) red_min(&a.reg[key].r, mine);
     return wmin < t;
+}
+template <bool kCoh>
+__device__ __forceinline__ ulonglong2 ld_reg(const RegSlot *p) {
+    return kCoh ? ld_gpu_slot(p) : ld_slot_ca(p);
+}
+
+// The keys of a range scan after its first (at most 15): their writer bits are
+// in one or two bitmap words, and only the keys with a writer are looked at
+// (2^18 x 10 scans of 10 keys: registration 73 -> 54 us; one dependent bitmap
+// load per key before).
+template <bool kCoh>
+__device__ __forceinline__ bool wf_read_rest(const YcsbTunedArgs &a, uint32_t w, uint32_t t,
+                                             uint32_t epoch) {
+    const uint32_t k1 = ycsb_key(w) + 1u, last = (uint32_t)scan_last(w, a.n);
+    if (last < k1) return false;  // a scan of the table's last key
+    const uint32_t lo = k1 >> 5, hi = last >> 5;
+    uint64_t win = ld_wbits<kCoh>(a.wbits + lo);
+    if (hi != lo) win |= (uint64_t)ld_wbits<kCoh>(a.wbits + hi) << 32;
+    uint32_t m = (uint32_t)(win >> (k1 & 31u)) & ((2u << (last - k1)) - 1u);
+    bool raw = false;
+    for (; m; m &= m - 1u) {
+        const uint32_t key = k1 + (uint32_t)__ffs(m) - 1u;
+        raw |= wf_read_key<kCoh>(a, key, t, epoch, ld_reg<kCoh>(a.reg + key));
+    }
+    return raw;
 }
 
 // The update list: the batch's u-th update (u = its value index, val_off[t]
@@ -414,9 +498,9 @@ __device__ __forceinline__ uint32_t vec_updates(const uint32_t *w) {
     for (int q = 0; q < 4; ++q) n += (!ycsb_is_pad(w[q]) && ycsb_is_update(w[q])) ? 1u : 0u;
     return n;
 }
-__device__ __forceinline__ void wf_list_updates(const YcsbTunedArgs &a, bool act, uint64_t v, uint32_t t,
+__device__ __forceinline__ void wf_list_updates(const YcsbTunedArgs &a, bool act, uint32_t v, uint32_t t,
                                                 const uint32_t *words) {
-    const uint32_t vpt = a.stride / 4u, seg = (uint32_t)(v % vpt);
+    const uint32_t vpt = a.stride / 4u, seg = act ? v - t * vpt : v % vpt;
     const bool pow2 = (vpt & (vpt - 1u)) == 0u;
     const uint32_t off = act ? __ldg(a.val_off + t) : 0u;
     const uint32_t end = act && seg == vpt - 1u ? __ldg(a.val_off + t + 1) : 0u;
@@ -454,18 +538,16 @@ __device__ __forceinline__ void wf_list_updates(const YcsbTunedArgs &a, bool act
 // wait behind the slot loads this pass is bound by.
 template <bool kCoh, bool kList = false>
 __device__ __forceinline__ void wf_register_reads(const YcsbTunedArgs &a, uint32_t epoch) {
-    const uint64_t tag = slot_tag(epoch);
-    const uint64_t nvec = (uint64_t)a.B * a.stride / 4u;
-    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+    const uint32_t vpt = a.stride / 4u, nvec = a.B * vpt;
+    const uint32_t step = gridDim.x * blockDim.x;
     const uint4 *vp = reinterpret_cast<const uint4 *>(a.ops);
     // a block-uniform loop, so that whole warps reach the warp-wide calls below
-    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < nvec; base += step) {
-        const uint64_t v = base + threadIdx.x;
+    for (uint32_t base = blockIdx.x * blockDim.x; base < nvec; base += step) {
+        const uint32_t v = base + threadIdx.x;
         const bool act = v < nvec;
         const uint4 w4 = act ? ld_nc_u4(vp + v)
                              : make_uint4(LTPG_YCSB_OP_PAD, LTPG_YCSB_OP_PAD, LTPG_YCSB_OP_PAD, LTPG_YCSB_OP_PAD);
-        const uint32_t t = act ? (uint32_t)(v * 4u / a.stride) : 0xFFFFFFFFu;
-        const unsigned long long mine = tag | t;
+        const uint32_t t = act ? v / vpt : 0xFFFFFFFFu;
         const uint32_t words[4] = {w4.x, w4.y, w4.z, w4.w};
         if (kList) wf_list_updates(a, act, v, t, words);
         bool rd[4];
@@ -480,21 +562,13 @@ __device__ __forceinline__ void wf_register_reads(const YcsbTunedArgs &a, uint32
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const uint32_t key = ycsb_key(words[q]);
-            s[q] = (bits[q] >> (key & 31u)) & 1u ? (kCoh ? ld_gpu_slot(a.reg + key) : ld_slot_ca(a.reg + key))
-                                                 : make_ulonglong2(~0ull, ~0ull);
+            s[q] = (bits[q] >> (key & 31u)) & 1u ? ld_reg<kCoh>(a.reg + key) : make_ulonglong2(~0ull, ~0ull);
         }
         bool raw = false;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const uint32_t w = words[q], key = ycsb_key(w);
-            const uint32_t wmin = slot_min(s[q].y, epoch);
-            if (wmin != 0xFFFFFFFFu && s[q].x > mine) red_min(&a.reg[key].r, mine);
-            raw |= wmin < t;
-            if (rd[q] && ycsb_span(w)) {  // a range scan: the keys after the first
-                const uint64_t last = scan_last(w, a.n);
-                for (uint64_t k2 = (uint64_t)key + 1; k2 <= last; ++k2)
-                    raw |= wf_read_key<kCoh>(a, k2, t, epoch, mine);
-            }
+            raw |= wf_read_key<kCoh>(a, ycsb_key(words[q]), t, epoch, s[q]);
+            if (rd[q] && ycsb_span(words[q])) raw |= wf_read_rest<kCoh>(a, words[q], t, epoch);
         }
         // one atomic per transaction: the lowest of its threads in the warp
         // ORs the bit when any of them saw RAW
@@ -571,8 +645,7 @@ __global__ void __launch_bounds__(BS) ycsb_wf_check_list(YcsbTunedArgs a) { wf_c
 // no third pass (the reads have a kernel of their own).  With late reads the
 // updates are stored by a later kernel.
 template <int kLate>
-__device__ __forceinline__ void checkwb_tiles(const YcsbTunedArgs &a, uint32_t *fl,
-                                              uint32_t epoch) {
+__device__ __forceinline__ void checkwb_tiles(const YcsbTunedArgs &a, uint32_t *fl, RowScratch *ws, uint32_t epoch) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t nvec_tile = a.tile * a.stride / 4;
     const uint32_t n_tiles = (a.B + a.tile - 1) / a.tile;
@@ -634,7 +707,7 @@ __device__ __forceinline__ void checkwb_tiles(const YcsbTunedArgs &a, uint32_t *
         // pass 3: committed updates, one thread per transaction in op order
         // (or, with late reads, the committed transactions' row reads)
         if (kLate == 1) {
-            late_read_tile(a, fl, t0, nt);
+            late_read_tile(a, ws, fl, t0, nt);
         } else if (kLate == 0) {
             for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x)
                 if (fl[i] & LTPG_FLAG_COMMIT) write_txn_updates(a, t0 + i);
@@ -781,15 +854,14 @@ __global__ void __launch_bounds__(BS) ycsb_exec_fast(YcsbTunedArgs a, uint32_t l
 // check, by the committed transactions alone (late_read_tile).
 template <bool kStage, bool kFilter, bool kDedupe, bool kReads>
 __device__ __forceinline__ void coop_exec_loop(const YcsbTunedArgs &a, StageEnt *tab, const uint32_t *sbits,
-                                               const uint32_t *srank, uint64_t tag) {
+                                               const uint32_t *srank, RowScratch *ws,
+                                               uint64_t tag) {
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t lanes_below = (1u << lane) - 1u;
     const uint32_t lpt = a.lpt;  // lanes per transaction, a power of two
     const uint32_t lsh = (uint32_t)__ffs(lpt) - 1u;
     const uint32_t groups = a.ways ? a.stage_entries / a.ways : 0u;
     const uint64_t nw = (uint64_t)a.B << lsh;
     const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
-    const uint32_t grp = lane / 5, chunk = lane % 5;  // row-read lane groups (6 x 5 lanes)
     bool scans = false;  // some read of this thread's was a range scan
     for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < nw; base += step) {
         const uint64_t v = base + threadIdx.x;
@@ -824,20 +896,11 @@ __device__ __forceinline__ void coop_exec_loop(const YcsbTunedArgs &a, StageEnt 
         if (kDedupe || kStage) peers = __match_any_sync(FULL, valid ? (key | (upd ? 0x80000000u : 0u)) : 0xFFFFFFFFu);
         const uint32_t leader_lane = (uint32_t)__ffs(peers) - 1u;
         const bool leader = valid && leader_lane == lane;
-        // rows still to read, compacted: round r reads the (6r + g)-th of them
+        // rows still to read
         const unsigned need = kReads ? __ballot_sync(FULL, rd && !have_dig && leader) : 0u;
-        const uint32_t n_need = __popc(need);
         ulonglong2 ch[6];
-#pragma unroll
-        for (int r = 0; r < 6; ++r) {
-            const uint32_t idx = (uint32_t)r * 6u + grp;
-            const bool go = kReads && grp < 6 && idx < n_need;
-            const uint32_t src = go ? __fns(need, 0, (int)idx + 1) : 0u;
-            const uint32_t k_src = __shfl_sync(FULL, key, src & 31u);
-            ch[r] = go ? ld_nc16_issue(reinterpret_cast<const char *>(a.rows + (uint64_t)k_src * LTPG_YCSB_FIELDS) +
-                                       16u * chunk)
-                       : make_ulonglong2(0ull, 0ull);
-        }
+        if (kReads && kStage) rows_issue_shfl(a.rows, key, need, ch);
+        else if (kReads && need) rows_issue(a.rows, ws, key, need, ch);  // warp-uniform
         // registration: staged rows in shared memory, the rest through the
         // warp dedupe and the slot filter
         const bool need_global = valid && !e;
@@ -852,21 +915,11 @@ __device__ __forceinline__ void coop_exec_loop(const YcsbTunedArgs &a, StageEnt 
         if (need_global && (kDedupe ? leader : true) && cur > mine) red_min_exec(slot, mine);
         scans |= rd && ycsb_span(w) != 0u;
         if (!kReads) continue;
-        // fold the five chunks of each row onto its group's first lane (5g),
-        // then hand the row's xor to the lane that owns the op
-        const uint32_t my_rank = __popc(need & lanes_below);
-#pragma unroll
-        for (int r = 0; r < 6; ++r) {
-            if ((uint32_t)r * 6u >= n_need) break;  // warp-uniform
-            const unsigned long long c0 = ch[r].x ^ ch[r].y;
-            unsigned long long c = c0 ^ __shfl_down_sync(FULL, c0, 1);  // lane 5g: chunks 0,1
-            c ^= __shfl_down_sync(FULL, c, 2);                          // lane 5g: chunks 0..3
-            const unsigned long long rowx = c ^ __shfl_down_sync(FULL, c0, 4);  // + chunk 4
-            const uint32_t op0 = (uint32_t)r * 6u;
-            const unsigned long long got = __shfl_sync(FULL, rowx, ((my_rank - op0) * 5u) & 31u);
-            if (((need >> lane) & 1u) && my_rank >= op0 && my_rank < op0 + 6u) x = got;
+        if (need) {
+            const unsigned long long rowx = kStage ? rows_fold_shfl(need, ch) : rows_fold(ws, need, ch);
+            if ((need >> lane) & 1u) x = rowx;
         }
-        {
+        if (kDedupe || kStage) {
             const unsigned long long from_leader = __shfl_sync(FULL, x, leader_lane);
             if (!have_dig) x = from_leader;
         }
@@ -950,7 +1003,7 @@ __global__ void __launch_bounds__(BS) ycsb_exec_coop(YcsbTunedArgs a) {
         stage_init(tab, a.stage_entries);
         __syncthreads();
     }
-    coop_exec_loop<kStage, kFilter, kDedupe, kReads>(a, tab, sbits, srank, tag);
+    coop_exec_loop<kStage, kFilter, kDedupe, kReads>(a, tab, sbits, srank, kReads && !kStage ? row_scratch<BS>() : nullptr, tag);
     if (kStage) {
         __syncthreads();
         const uint32_t ops = stage_flush(tab, a.stage_entries, a.reg, tag, a.bucket_counts);
@@ -1002,7 +1055,7 @@ template <int kLate>
 __global__ void __launch_bounds__(512) ycsb_checkwb_tuned(YcsbTunedArgs a) {
     extern __shared__ __align__(16) char smem[];
     const SmemPtrs p = carve(smem, a.tile);
-    checkwb_tiles<kLate>(a, p.fl, a.ctl->epoch);
+    checkwb_tiles<kLate>(a, p.fl, kLate == 1 ? row_scratch<512>() : nullptr, a.ctl->epoch);
     if (!kLate) finish_batch<false>(a.ctl);
 }
 
@@ -1095,10 +1148,11 @@ __global__ void __launch_bounds__(BS) ycsb_writeback_list(YcsbTunedArgs a) {
 // then check + reads, a second grid barrier, and the write-back.  Phases
 // after the first load what earlier phases wrote with coherent loads
 // (kCoh = true above; checkwb_tiles reads slots with ld.global.cg, at L2).
-template <bool kStage, bool kLate>
+template <bool kStage, bool kLate, int BS>
 __device__ __forceinline__ void ycsb_persistent_body(const YcsbTunedArgs &a) {
     extern __shared__ __align__(16) char smem[];
     const SmemPtrs p = carve(smem, a.tile);
+    RowScratch *ws = row_scratch<BS>();
     const uint32_t epoch = a.ctl->epoch;
     const uint64_t tag = slot_tag(epoch);
     if (kLate && !kStage && a.late == 3u) {  // write-first: five phases, four grid barriers
@@ -1108,7 +1162,7 @@ __device__ __forceinline__ void ycsb_persistent_body(const YcsbTunedArgs &a) {
         ok = ok && grid_barrier(a.ctl);
         if (ok) wf_check_list<true>(a, epoch);
         ok = ok && grid_barrier(a.ctl);
-        if (ok) late_read_loop<true>(a);
+        if (ok) late_read_loop<true>(a, ws);
         ok = ok && grid_barrier(a.ctl);
         if (ok) writeback_list<true>(a);
         if (ok) finish_batch<false>(a.ctl);
@@ -1120,8 +1174,8 @@ __device__ __forceinline__ void ycsb_persistent_body(const YcsbTunedArgs &a) {
         __syncthreads();
     }
     if (a.lpt) {
-        if (a.filter) coop_exec_loop<kStage, true, true, !kLate>(a, p.tab, a.stage_bits, a.stage_rank, tag);
-        else coop_exec_loop<kStage, false, true, !kLate>(a, p.tab, a.stage_bits, a.stage_rank, tag);
+        if (a.filter) coop_exec_loop<kStage, true, true, !kLate>(a, p.tab, a.stage_bits, a.stage_rank, ws, tag);
+        else coop_exec_loop<kStage, false, true, !kLate>(a, p.tab, a.stage_bits, a.stage_rank, ws, tag);
     } else if (!kLate) {
         exec_tiles<kStage>(a, p.dig, p.tab, tag);
     }
@@ -1132,14 +1186,14 @@ __device__ __forceinline__ void ycsb_persistent_body(const YcsbTunedArgs &a) {
     }
     bool ok = grid_barrier(a.ctl);
     if (ok) {
-        if (!kLate) checkwb_tiles<0>(a, p.fl, epoch);
-        else if (a.late == 2u) checkwb_tiles<2>(a, p.fl, epoch);
-        else checkwb_tiles<1>(a, p.fl, epoch);
+        if (!kLate) checkwb_tiles<0>(a, p.fl, ws, epoch);
+        else if (a.late == 2u) checkwb_tiles<2>(a, p.fl, ws, epoch);
+        else checkwb_tiles<1>(a, p.fl, ws, epoch);
     }
     if (kLate) {
         if (a.late == 2u) {
             ok = ok && grid_barrier(a.ctl);
-            if (ok) late_read_loop<true>(a);
+            if (ok) late_read_loop<true>(a, ws);
         }
         ok = ok && grid_barrier(a.ctl);
         if (ok) writeback_late_loop<false, true>(a);
@@ -1148,13 +1202,15 @@ __device__ __forceinline__ void ycsb_persistent_body(const YcsbTunedArgs &a) {
     else finish_batch(a.ctl);
 }
 template <bool kStage, bool kLate>
-__global__ void __launch_bounds__(512) ycsb_persistent(YcsbTunedArgs a) { ycsb_persistent_body<kStage, kLate>(a); }
+__global__ void __launch_bounds__(512) ycsb_persistent(YcsbTunedArgs a) {
+    ycsb_persistent_body<kStage, kLate, 512>(a);
+}
 // Late reads on blocks of at most 256 threads with registers budgeted for six
 // resident blocks per SM (40, with a few spills, against 59 and four): the row
 // gathers of the late-read phase want the warps more than the other phases
 // want the registers.
 __global__ void __launch_bounds__(256, 6) ycsb_persistent_late_x6(YcsbTunedArgs a) {
-    ycsb_persistent_body<false, true>(a);
+    ycsb_persistent_body<false, true, 256>(a);
 }
 
 // Static shared memory of a kernel, queried once per kernel.
