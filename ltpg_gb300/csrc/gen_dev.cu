@@ -5,9 +5,10 @@
 // Compiled with -fmad=false: the Zipf sampler's double arithmetic (gen.h) must
 // round exactly like the host's.
 //
-// YCSB: one thread per transaction draws its op words (gen::ycsb_txn), an
-// inclusive scan of the update counts gives val_off, and one thread per
-// transaction writes its update values.
+// YCSB: a block draws the keys of a tile of transactions one operation per
+// thread, redraws the repeated ones until none is left (ycsb_gen_ops), an
+// inclusive scan of the update counts gives val_off, and one lane per operation
+// writes its update's value.
 //
 // TPC-C: the host generator is a loop whose per-warehouse counters (O_ID,
 // NO_ID, OL_ID, H_ID) and order memory (for OrderStatus and Delivery) carry
@@ -42,6 +43,7 @@ constexpr uint32_t TB = 256;          // threads per block of the per-transactio
 constexpr uint32_t SCAN_T = 1024;     // threads per block of the scan
 constexpr uint32_t SCAN_V = 4;        // values per scan thread
 constexpr uint32_t SCAN_BLOCK = SCAN_T * SCAN_V;
+constexpr uint32_t SCAN_DIRECT = 1024;  // up to this many block totals are summed by their users
 constexpr uint32_t DL_TRACKED = 0x80000000u;
 constexpr uint64_t MAX_CHUNK_COUNTERS = 8ull << 20;  // per class, chunks x warehouses
 
@@ -139,33 +141,238 @@ uint32_t scan_scratch(uint32_t n) { return (n + SCAN_BLOCK - 1) / SCAN_BLOCK + 1
 // ---- YCSB ----------------------------------------------------------------------
 struct YcsbGenArgs {
     ltpg_ycsb_params p;
-    Zipf zipf;
+    FastZipf zipf;
     const FixTables *tab;
+    const PolyCell *cells;
     Perm perm;
     bool rotate;
     uint64_t batch_id;
     uint32_t *ops, *val_off;
     uint64_t *vals;
+    uint32_t tile;         // slots of a warp
+    uint32_t k_inv, s_inv; // ceil(2^16 / k), ceil(2^16 / stride): i / k = i k_inv >> 16 for a tile's indices
 };
 
-__global__ void __launch_bounds__(TB) ycsb_gen_ops(YcsbGenArgs a) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t == 0) a.val_off[0] = 0;
-    if (t >= a.p.n_txn) return;
-    const uint32_t stride = ycsb_stride(a.p.ops_per_txn);
-    a.val_off[t + 1] =
-        ycsb_txn(a.p, a.zipf, *a.tab, a.rotate ? &a.perm : nullptr, a.batch_id, t, a.ops + (uint64_t)t * stride);
+// Draw number d (0-based) of the stream that starts at state s.
+__device__ __forceinline__ uint64_t draw_at(uint64_t s, uint32_t d) {
+    Rng r(s + (uint64_t)d * 0x9E3779B97F4A7C15ull);
+    return r.next();
 }
 
-__global__ void __launch_bounds__(TB) ycsb_gen_vals(YcsbGenArgs a) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= a.p.n_txn) return;
-    const uint32_t k = a.p.ops_per_txn, stride = ycsb_stride(k);
-    const uint64_t txn = a.batch_id * (uint64_t)a.p.n_txn + t;
-    uint32_t v = a.val_off[t];
-    const uint32_t *w = a.ops + (uint64_t)t * stride;
-    for (uint32_t j = 0; j < k; ++j)
-        if (ycsb_is_update(w[j])) a.vals[v++] = ycsb_value(a.p, txn, j);
+// Op words of a batch, the bytes of ycsb_txn.  A transaction's draws are a
+// counter-based stream: operation j takes three (key, update?, field) from draw
+// 3j + (redraws so far), a redraw one more.  A warp holds up to 32 transactions
+// (256 words) in slots and repeats:
+//   1. free slots take the block's next transactions;
+//   2. every key not yet settled is drawn, one operation per lane, from a list:
+//      all of a new transaction's, as if none repeated, and of an old one's
+//      those from its first repeated key on, one draw up;
+//   3. each drawn key is compared with its transaction's earlier ones; a
+//      transaction without a repeat gets its update and field bits, its words
+//      are stored (coalesced), and its slot is free.
+// At theta = 0.99 over 10 M keys 45 % of the 16-op transactions repeat a key and
+// the redrawn operations are 20 % of all; refilling the slots keeps the lists
+// long (a thread per transaction ran as long as the warp's unluckiest lane; a
+// tile finished before the next was begun ran half-empty passes for its last
+// repeats, 146 us per 2^18 transactions against 120).  A transaction still
+// repeating after GEN_ROUNDS rounds (tiny tables, whose walk to a free key
+// starts at the 65th draw of an operation) is made by ycsb_txn, alone.  The hot
+// set's permutation, four rounds of a hash of at most 12 bits for up to 2^24
+// keys, is tabulated by the block (4 x 2^half entries of 16 bits).  2^20 x 16
+// ops, theta 0.99: 1006 us one thread per transaction, 350 us now; bound by the
+// integer pipes.
+constexpr uint32_t GEN_T = 512, GEN_WORDS = 256, GEN_ROUNDS = 16, PERM_HALF = 12;
+constexpr uint32_t PERM_BYTES = (4u << PERM_HALF) * sizeof(uint16_t);
+
+struct __align__(16) GenSlots {
+    uint64_t seed[32];            // stream state of each slot's transaction
+    uint32_t first[32];           // its first repeated key (k: none)
+    uint32_t redraws[32];
+    uint32_t cnt[32];             // updates
+    uint32_t key[GEN_WORDS];      // by word: slot * stride + j
+    uint8_t shift[GEN_WORDS];     // by word: redraws up to and with the operation
+    uint8_t list[GEN_WORDS];      // operations to draw, slot * k + j
+    uint8_t settled[32];          // slots to store
+    uint64_t pad[2];
+};
+constexpr uint32_t GEN_BYTES = POLY_CELLS * sizeof(PolyCell) + GEN_T / 32 * sizeof(GenSlots);  // + the permutation
+
+__global__ void __launch_bounds__(GEN_T, 2) ycsb_gen_ops(YcsbGenArgs a) {
+    extern __shared__ __align__(16) char gen_smem[];
+    PolyCell *cells = reinterpret_cast<PolyCell *>(gen_smem);
+    GenSlots *slots = reinterpret_cast<GenSlots *>(cells + POLY_CELLS);
+    uint16_t *perm_tab = reinterpret_cast<uint16_t *>(slots + GEN_T / 32);  // [4][2^half] when tabulated
+    __shared__ uint32_t next;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, k = a.p.ops_per_txn, stride = ycsb_stride(k), B = a.p.n_txn;
+    const uint32_t half = a.perm.half, mask = (1u << half) - 1u, span = a.p.scan_len >= 2u ? a.p.scan_len - 1u : 0u;
+    const bool tabulated = a.rotate && half <= PERM_HALF;
+    if (a.zipf.fast)
+        for (uint32_t i = tid; i < POLY_CELLS * sizeof(PolyCell) / 16u; i += GEN_T)
+            reinterpret_cast<uint4 *>(cells)[i] = reinterpret_cast<const uint4 *>(a.cells)[i];
+    if (tabulated)
+        for (uint32_t i = tid; i < (4u << half); i += GEN_T)
+            perm_tab[i] = (uint16_t)a.perm.round_fn(i & mask, i >> half);
+    if (blockIdx.x == 0 && tid == 0) a.val_off[0] = 0;
+    // the block's transactions: [begin, end)
+    const uint32_t end = (uint32_t)((uint64_t)B * (blockIdx.x + 1u) / gridDim.x);
+    if (tid == 0) next = (uint32_t)((uint64_t)B * blockIdx.x / gridDim.x);
+    __syncthreads();
+
+    GenSlots &g = slots[tid >> 5];
+    bool active = false;  // this lane's slot holds a transaction
+    uint32_t t = 0, from = 0;
+    for (;;) {
+        // 1. refill
+        const unsigned free = __ballot_sync(0xFFFFFFFFu, lane < a.tile && !active);
+        uint32_t base = 0;
+        if (lane == 0u) base = atomicAdd(&next, __popc(free));
+        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+        if ((free >> lane) & 1u) {
+            t = base + __popc(free & ((1u << lane) - 1u));
+            active = base < end && t < end;
+            from = 0;
+            if (active) {
+                g.seed[lane] = hash3(a.p.seed ^ DOM_YCSB_OPS, a.batch_id, t);
+                g.redraws[lane] = 0u;
+                g.cnt[lane] = 0u;
+            }
+        }
+        if (!__any_sync(0xFFFFFFFFu, active)) break;
+        // 2. the keys to draw, then the draws
+        const uint32_t m = active ? k - from : 0u, incl = warp_scan_incl(m);
+        const uint32_t n = __shfl_sync(0xFFFFFFFFu, incl, 31);
+        if (active) {
+            for (uint32_t j = from; j < k; ++j) g.list[incl - k + j] = (uint8_t)(lane * k + j);
+            g.first[lane] = k;
+        }
+        __syncwarp();
+        for (uint32_t e = lane; e < n; e += 32u) {
+            const uint32_t i = g.list[e], lt = i * a.k_inv >> 16, j = i - lt * k, s = g.redraws[lt];
+            uint64_t y = fast_sample(a.zipf, cells, *a.tab, draw_at(g.seed[lt], 3u * j + s));
+            if (tabulated) {
+                uint32_t l = (uint32_t)(y >> half), r = (uint32_t)y & mask;
+                do {
+#pragma unroll
+                    for (uint32_t f = 0; f < 4; ++f) {
+                        const uint32_t x = l ^ perm_tab[(f << half) + r];
+                        l = r;
+                        r = x;
+                    }
+                } while (((l << half) | r) >= (uint32_t)a.perm.n);
+                y = (l << half) | r;
+            } else if (a.rotate) {
+                y = a.perm(y);
+            }
+            g.key[lt * stride + j] = (uint32_t)y;
+            g.shift[lt * stride + j] = (uint8_t)s;
+        }
+        __syncwarp();
+        // 3. repeats
+        for (uint32_t e = lane; e < n; e += 32u) {
+            const uint32_t i = g.list[e], lt = i * a.k_inv >> 16, j = i - lt * k;
+            const uint32_t *row = g.key + lt * stride, key = row[j];
+            bool dup = false;
+            uint32_t q = 0;
+            for (; q + 3u < j; q += 4u) {
+                const uint4 w = *reinterpret_cast<const uint4 *>(row + q);
+                dup |= w.x == key | w.y == key | w.z == key | w.w == key;
+            }
+            for (; q < j; ++q) dup |= row[q] == key;
+            if (dup) atomicMin(&g.first[lt], j);
+        }
+        __syncwarp();
+        bool settled = false;
+        if (active) {
+            from = g.first[lane];
+            settled = from == k;
+            if (!settled && ++g.redraws[lane] > GEN_ROUNDS) {
+                uint32_t w[LTPG_YCSB_MAX_OPS];
+                const uint32_t nu = ycsb_txn(a.p, a.zipf.z, *a.tab, a.rotate ? &a.perm : nullptr, a.batch_id, t, w);
+                for (uint32_t j = 0; j < stride; ++j) a.ops[(uint64_t)t * stride + j] = w[j];
+                a.val_off[t + 1u] = nu;
+                active = false;
+            }
+        }
+        const unsigned done = __ballot_sync(0xFFFFFFFFu, settled);
+        if (settled) g.settled[__popc(done & ((1u << lane) - 1u))] = (uint8_t)lane;
+        __syncwarp();
+        const uint32_t words = __popc(done) * stride;
+        for (uint32_t v0 = 0; v0 < words; v0 += 32u) {  // whole warps: the shuffle below
+            const uint32_t v = v0 + lane, at = v < words ? v * a.s_inv >> 16 : 0u, j = v - at * stride;
+            const uint32_t lt = g.settled[at], tt = __shfl_sync(0xFFFFFFFFu, t, lt);
+            if (v >= words) continue;
+            uint32_t w = LTPG_YCSB_OP_PAD;
+            if (j < k) {
+                const uint32_t d = 3u * j + g.shift[lt * stride + j];
+                const bool upd = mulhi64(draw_at(g.seed[lt], d + 1u), 100u) < a.p.update_pct;
+                uint32_t field = span;
+                if (upd) {
+                    field = (uint32_t)mulhi64(draw_at(g.seed[lt], d + 2u), LTPG_YCSB_FIELDS);
+                    atomicAdd(&g.cnt[lt], 1u);
+                }
+                w = ycsb_word(g.key[lt * stride + j], upd, field);
+            }
+            a.ops[(uint64_t)tt * stride + j] = w;
+        }
+        __syncwarp();
+        if (settled) {
+            a.val_off[t + 1u] = g.cnt[lane];
+            active = false;
+        }
+        __syncwarp();
+    }
+}
+
+// Update values, and the value offsets completed: val_off[t + 1] holds the
+// update count of transaction t's SCAN_BLOCK so far, blk[c] the total of block
+// c.  A block of threads stays inside one SCAN_BLOCK and sums the totals before
+// it; a warp takes 32 / (stride / 4) whole transactions at a time, four words
+// per lane, and a lane's first value index is the count of its transaction's
+// updates in the earlier lanes.
+__global__ void __launch_bounds__(TB) ycsb_gen_vals(YcsbGenArgs a, const uint32_t *blk, bool scanned) {
+    __shared__ uint32_t part[TB / 32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t B = a.p.n_txn, vpt = ycsb_stride(a.p.ops_per_txn) / 4u, tpw = 32u / vpt;
+    const uint32_t t_begin = blockIdx.x * TB, t_end = min(B, t_begin + TB), c = t_begin / SCAN_BLOCK;
+    uint32_t before = 0;
+    if (scanned) {  // blk holds inclusive sums
+        before = c ? blk[c - 1u] : 0u;
+    } else {
+        for (uint32_t i = threadIdx.x; i < c; i += TB) before += blk[i];
+        before = __reduce_add_sync(0xFFFFFFFFu, before);
+        if (lane == 0u) part[warp] = before;
+        __syncthreads();
+        before = 0;
+        for (uint32_t i = 0; i < TB / 32; ++i) before += part[i];
+    }
+    const uint32_t lt = lane / vpt, seg = lane - lt * vpt;
+    const uint4 *vp = reinterpret_cast<const uint4 *>(a.ops);
+    for (uint32_t t0 = t_begin + warp * tpw; t0 < t_end; t0 += (TB / 32) * tpw) {
+        const uint32_t t = t0 + lt;
+        const bool act = lt < tpw && t < t_end;
+        const uint4 w4 = act ? vp[(uint64_t)t * vpt + seg]
+                             : make_uint4(LTPG_YCSB_OP_PAD, LTPG_YCSB_OP_PAD, LTPG_YCSB_OP_PAD, LTPG_YCSB_OP_PAD);
+        const uint32_t end = act ? a.val_off[t + 1] + before : 0u;
+        const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
+        uint32_t n = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) n += !ycsb_is_pad(w[q]) && ycsb_is_update(w[q]);
+        uint32_t incl = n;  // over the transaction's lanes so far
+        for (uint32_t o = 1; o < vpt; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (seg >= o) incl += y;
+        }
+        const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, (lt * vpt + vpt - 1u) & 31u);
+        uint32_t v = end - total + incl - n;
+        if (n) {  // ycsb_value, its part that the transaction's operations share made once
+            const uint64_t h = splitmix64(splitmix64(a.p.seed ^ DOM_YCSB_VAL) ^ (a.batch_id * (uint64_t)B + t));
+#pragma unroll
+            for (uint32_t q = 0; q < 4; ++q)
+                if (!ycsb_is_pad(w[q]) && ycsb_is_update(w[q])) a.vals[v++] = splitmix64(h ^ (4u * seg + q));
+        }
+        // every lane of the transaction has read its count by the shuffle above
+        if (act && seg == 0u) a.val_off[t + 1] = end;
+    }
 }
 
 // ---- TPC-C ---------------------------------------------------------------------
@@ -466,6 +673,9 @@ uint32_t blocks(uint64_t n, uint32_t per) { return (uint32_t)((n + per - 1) / pe
 struct ltpg_gen_dev {
     int device = -1;
     FixTables *tab = nullptr;
+    PolyCell *cells = nullptr;
+    FastZipf zipf;
+    uint32_t gen_blocks = 0;  // resident blocks of ycsb_gen_ops on the device
     uint32_t G = 0, C = 0;
     uint32_t *o_id = nullptr, *no_id = nullptr, *ol_id = nullptr, *h_id = nullptr;
     uint64_t *made = nullptr, *delivered = nullptr;
@@ -563,8 +773,18 @@ cudaError_t bind_ycsb(ltpg_gen *g, int device) {
     ltpg_gen_dev *d = new (std::nothrow) ltpg_gen_dev();
     if (!d) return cudaErrorMemoryAllocation;
     d->device = device;
+    std::vector<PolyCell> cells(POLY_CELLS);
+    d->zipf = fast_zipf(g->zipf, cells.data());
     cudaError_t e = dalloc(d, &d->tab, 1);
     if (e == cudaSuccess) e = cudaMemcpy(d->tab, &host_fix_tables(), sizeof(FixTables), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = dput(d, &d->cells, cells);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(ycsb_gen_ops, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(GEN_BYTES + PERM_BYTES));
+    int per_sm = 0, sms = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ycsb_gen_ops, GEN_T, GEN_BYTES + PERM_BYTES);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    d->gen_blocks = (uint32_t)(std::max(per_sm, 1) * std::max(sms, 1));
     if (e != cudaSuccess) {
         free_dev(d);
         return e;
@@ -599,28 +819,33 @@ int gen_ycsb(ltpg_ctx *c, ltpg_gen *g, uint64_t batch_id, uint32_t slot, cudaStr
     if (!g->dev && (e0 = bind_ycsb(g, c->device)) != cudaSuccess) return ctx_cuda_fail(c, e0, "generator tables");
     YcsbGenArgs a;
     a.p = p;
-    a.zipf = g->zipf;
+    a.zipf = g->dev->zipf;
     a.tab = g->dev->tab;
+    a.cells = g->dev->cells;
     a.rotate = p.rotate_every != 0;
     if (a.rotate) a.perm.init(p.n_records, hash3(p.seed ^ DOM_YCSB_PERM, batch_id / p.rotate_every, 0));
     a.batch_id = batch_id;
     a.ops = s->ops;
     a.val_off = s->val_off;
     a.vals = s->vals;
-    const uint32_t nb = blocks(p.n_txn, TB);
-    ycsb_gen_ops<<<nb, TB, 0, st>>>(a);
+    const uint32_t stride = ycsb_stride(p.ops_per_txn), warps = g->dev->gen_blocks * (GEN_T / 32);
+    // slots as the shared arrays take them, fewer while some warps would get no transaction
+    a.tile = std::min(std::min<uint32_t>(32, GEN_WORDS / stride), std::max<uint32_t>(2, blocks(p.n_txn, warps)));
+    a.k_inv = (65536u + p.ops_per_txn - 1) / p.ops_per_txn;
+    a.s_inv = (65536u + stride - 1) / stride;
+    const uint32_t perm_bytes = a.rotate && a.perm.half <= PERM_HALF ? (4u << a.perm.half) * sizeof(uint16_t) : 0u;
+    ycsb_gen_ops<<<std::min(blocks(blocks(p.n_txn, a.tile), GEN_T / 32), g->dev->gen_blocks), GEN_T, GEN_BYTES + perm_bytes,
+                   st>>>(a);
     count_launch(c);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) {
-        // the scan's block totals borrow the slot's vals buffer, whose values
-        // are written after the scan
-        uint64_t launches = 0;
-        e = inclusive_scan(s->val_off + 1, p.n_txn, reinterpret_cast<uint32_t *>(s->vals), st, launches);
-        count_launch(c, launches);
-    }
-    if (e == cudaSuccess) {
-        ycsb_gen_vals<<<nb, TB, 0, st>>>(a);
-        count_launch(c);
+        const uint32_t nb = blocks(p.n_txn, SCAN_BLOCK);
+        uint32_t *blk = s->off_blocks;
+        const bool scanned = nb > SCAN_DIRECT;
+        scan_blocks<<<nb, SCAN_T, 0, st>>>(s->val_off + 1, p.n_txn, blk);
+        if (scanned) scan_totals<<<1, SCAN_T, 0, st>>>(blk, nb);
+        ycsb_gen_vals<<<blocks(p.n_txn, TB), TB, 0, st>>>(a, blk, scanned);
+        count_launch(c, scanned ? 3 : 2);
         e = cudaGetLastError();
     }
     return e == cudaSuccess ? LTPG_OK : ctx_cuda_fail(c, e, "device YCSB generation");
