@@ -223,7 +223,9 @@ int ltpg_gen_tpcc_batch(ltpg_gen *g, uint64_t batch_id, ltpg_tpcc_txn *txns,
             g->no_id[w] = (g->no_id[w] + 1) % 30000u;
             x.c = g->ol_id[w];
             g->ol_id[w] = (g->ol_id[w] + h.cnt) % 450000u;
-            tpcc_neworder(p, r, h, x, lines + nl);
+            tpcc_neworder(
+                p, r, h, x, [&](uint32_t i, const ltpg_tpcc_line &ln) { lines[nl + i] = ln; },
+                [&](uint32_t i) { return lines[nl + i].i_id; });
             if (tracking) {
                 const size_t k = 30000ull * w + x.a;
                 g->o_cust[k] = (uint16_t)x.c_id;

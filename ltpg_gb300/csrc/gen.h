@@ -491,9 +491,11 @@ LTPG_HDI void tpcc_by_name(const ltpg_tpcc_params &p, Rng &r, ltpg_tpcc_txn &x, 
 }
 
 // NewOrder after its head: customer, then the lines (distinct items within an
-// order, TF/Query.h:103-114).  O_ID / NO_ID / first OL_ID are the caller's.
-LTPG_HDI void tpcc_neworder(const ltpg_tpcc_params &p, Rng &r, const TpccHead &h, ltpg_tpcc_txn &x,
-                            ltpg_tpcc_line *lines) {
+// order, TF/Query.h:103-114).  O_ID / NO_ID / first OL_ID are the caller's, as
+// is where the lines go: put(i, line), and item(i) gives line i's item back.
+template <class Put, class Item>
+LTPG_HDI void tpcc_neworder(const ltpg_tpcc_params &p, Rng &r, const TpccHead &h, ltpg_tpcc_txn &x, Put put,
+                            Item item_of) {
     x.kind_info = LTPG_TPCC_NEWORDER | (h.cnt << 8) | (h.d << 16);
     x.c_w = h.w;
     x.c_id = (uint32_t)nurand(r, 1023, 1, 3000) - 1;
@@ -502,7 +504,7 @@ LTPG_HDI void tpcc_neworder(const ltpg_tpcc_params &p, Rng &r, const TpccHead &h
         for (;;) {
             item = (uint32_t)nurand(r, 8191, 1, 100000) - 1;
             bool dup = false;
-            for (uint32_t q = 0; q < i; ++q) dup |= lines[q].i_id == item;
+            for (uint32_t q = 0; q < i; ++q) dup |= item_of(q) == item;
             if (!dup) break;
         }
         ltpg_tpcc_line ln;
@@ -510,7 +512,7 @@ LTPG_HDI void tpcc_neworder(const ltpg_tpcc_params &p, Rng &r, const TpccHead &h
         const bool remote = p.warehouses > 1 && r.below(100) < p.remote_line_pct;
         ln.supply_w = (uint16_t)(remote ? other_w(r, h.w, p.warehouses) : h.w);
         ln.qty = (uint16_t)r.range(1, 10);
-        lines[i] = ln;
+        put(i, ln);
     }
 }
 

@@ -23,8 +23,8 @@
 //      Payments, Deliveries) of its warehouse; each warehouse's NewOrders and
 //      Deliveries listed in batch order;
 //   5. NewOrder, Payment and StockLevel records;
-//   6. Delivery's oldest-undelivered counter, the only true recurrence: one
-//      sequential walk per warehouse over its Deliveries;
+//   6. Delivery's oldest-undelivered counter, the only true recurrence: a scan
+//      of its steps, which compose, per warehouse;
 //   7. OrderStatus and Delivery records, each remembered order read from the
 //      batch's NewOrder that made it or from the order memory at batch start;
 //   8. state: counters, order memory (last writer of each O_ID), slot header.
@@ -114,10 +114,22 @@ __global__ void __launch_bounds__(SCAN_T) scan_totals(uint32_t *blk, uint32_t nb
         __syncthreads();
     }
 }
-// Pass 3: block b adds the totals of blocks 0 .. b-1.
-__global__ void __launch_bounds__(SCAN_T) scan_add(uint32_t *a, uint32_t n, const uint32_t *blk) {
+// Pass 3: block b adds the totals of blocks 0 .. b-1: the inclusive sum that
+// pass 2 left, or (up to SCAN_DIRECT blocks, with no pass 2) summed here.
+__global__ void __launch_bounds__(SCAN_T) scan_add(uint32_t *a, uint32_t n, const uint32_t *blk, bool scanned) {
     if (blockIdx.x == 0) return;
-    const uint32_t add = blk[blockIdx.x - 1];
+    __shared__ uint32_t sh[32];
+    uint32_t add = 0;
+    if (scanned) {
+        add = blk[blockIdx.x - 1];
+    } else {
+        const uint32_t lane = threadIdx.x & 31u;
+        for (uint32_t i = threadIdx.x; i < blockIdx.x; i += SCAN_T) add += blk[i];
+        add = __reduce_add_sync(0xFFFFFFFFu, add);
+        if (lane == 0u) sh[threadIdx.x >> 5] = add;
+        __syncthreads();
+        add = __reduce_add_sync(0xFFFFFFFFu, sh[lane]);
+    }
     const uint64_t base = (uint64_t)blockIdx.x * SCAN_BLOCK + (uint64_t)threadIdx.x * SCAN_V;
 #pragma unroll
     for (uint32_t j = 0; j < SCAN_V; ++j)
@@ -127,12 +139,16 @@ __global__ void __launch_bounds__(SCAN_T) scan_add(uint32_t *a, uint32_t n, cons
 cudaError_t inclusive_scan(uint32_t *a, uint32_t n, uint32_t *blk, cudaStream_t st, uint64_t &launches) {
     if (n == 0) return cudaSuccess;
     const uint32_t nb = (n + SCAN_BLOCK - 1) / SCAN_BLOCK;
+    const bool scanned = nb > SCAN_DIRECT;
     scan_blocks<<<nb, SCAN_T, 0, st>>>(a, n, blk);
     ++launches;
-    if (nb > 1) {
+    if (scanned) {
         scan_totals<<<1, SCAN_T, 0, st>>>(blk, nb);
-        scan_add<<<nb, SCAN_T, 0, st>>>(a, n, blk);
-        launches += 2;
+        ++launches;
+    }
+    if (nb > 1) {
+        scan_add<<<nb, SCAN_T, 0, st>>>(a, n, blk, scanned);
+        ++launches;
     }
     return cudaGetLastError();
 }
@@ -436,20 +452,33 @@ __global__ void __launch_bounds__(TB) tpcc_gen_head(TpccGenArgs a) {
     }
 }
 
-// 3a. One warp per (class, warehouse): exclusive scan of its chunk counters.
+// 3a. One block per (class, warehouse): exclusive scan of its chunk counters.
 __global__ void __launch_bounds__(TB) tpcc_gen_chunk_scan(TpccGenArgs a) {
-    const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
-    if (gw >= 4u * a.W) return;
-    uint32_t *c = a.cc + (uint64_t)gw * a.G;
+    __shared__ uint32_t part[TB / 32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t *c = a.cc + (uint64_t)blockIdx.x * a.G;
     uint32_t carry = 0;
-    for (uint32_t g0 = 0; g0 < a.G; g0 += 32) {
-        const uint32_t g = g0 + lane;
-        const uint32_t v = g < a.G ? c[g] : 0u;
-        const uint32_t incl = warp_scan_incl(v);
-        if (g < a.G) c[g] = carry + incl - v;
-        carry += __shfl_sync(0xFFFFFFFFu, incl, 31);
+    for (uint32_t g0 = 0; g0 < a.G; g0 += TB * 4u) {
+        const uint32_t g = g0 + threadIdx.x * 4u;
+        uint32_t v[4], sum = 0;
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) sum += v[i] = g + i < a.G ? c[g + i] : 0u;
+        const uint32_t incl = warp_scan_incl(sum);
+        if (lane == 31u) part[warp] = incl;
+        __syncthreads();
+        uint32_t before = carry + incl - sum;
+        for (uint32_t i = 0; i < TB / 32; ++i) {
+            before += i < warp ? part[i] : 0u;
+            carry += part[i];
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+            if (g + i < a.G) c[g + i] = before;
+            before += v[i];
+        }
+        __syncthreads();
     }
-    if (lane == 0) a.tot[gw] = carry;
+    if (threadIdx.x == 0) a.tot[blockIdx.x] = carry;
 }
 
 // 3b. One block: list starts of each warehouse's NewOrders and Deliveries.
@@ -483,9 +512,12 @@ __global__ void __launch_bounds__(SCAN_T) tpcc_gen_starts(TpccGenArgs a) {
 }
 
 // 4. One warp per chunk, 32 transactions per step in batch order.  A lane
-// counts the step's earlier lanes of its warehouse by shuffles; the
-// warehouse's running counters of the chunk (the chunk counters, now
-// prefixes) are advanced by the step's last lane of that warehouse.
+// counts the step's earlier lanes of its warehouse by ballots (its peers by one
+// match; line counts bit by bit); the warehouse's running counters of the chunk
+// (the chunk counters, now prefixes) are advanced by the step's last lane of
+// that warehouse.  Steps follow one another through those counters, so chunks
+// are short: 128 transactions (W = 64, 2^18: 102 us with 1,024 and a shuffle
+// per earlier lane, 16 us now).
 //   nob[t]  NewOrders of w before t in the batch (every kind)
 //   aux[t]  NewOrder: lines of w's earlier NewOrders; Payment: earlier
 //           Payments of w; Delivery: earlier Deliveries of w
@@ -496,28 +528,19 @@ __global__ void __launch_bounds__(TB) tpcc_gen_rank(TpccGenArgs a) {
     for (uint32_t base = g * a.C; base < t_end; base += 32) {
         const uint32_t t = base + lane;
         const bool valid = t < t_end;
-        TpccHead h{0u, 0xFFFFFFFFu, 0u, 0u};
+        TpccHead h{0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u};
         if (valid) {
             Rng r = tpcc_rng(a, t);
             h = tpcc_head(a.p, r);
         }
-        const uint32_t key = valid ? h.w : 0xFFFFFFFFu;
-        uint32_t pno = 0, pol = 0, ppay = 0, pdl = 0;
-        bool last = valid;
-        for (uint32_t src = 0; src < 32; ++src) {
-            const uint32_t kw = __shfl_sync(0xFFFFFFFFu, key, src);
-            const uint32_t kk = __shfl_sync(0xFFFFFFFFu, h.kind, src);
-            const uint32_t kc = __shfl_sync(0xFFFFFFFFu, h.cnt, src);
-            if (kw != key || !valid) continue;
-            if (src < lane) {
-                pno += kk == LTPG_TPCC_NEWORDER;
-                pol += kk == LTPG_TPCC_NEWORDER ? kc : 0u;
-                ppay += kk == LTPG_TPCC_PAYMENT;
-                pdl += kk == LTPG_TPCC_DELIVERY;
-            } else if (src > lane) {
-                last = false;
-            }
-        }
+        const unsigned peers = __match_any_sync(0xFFFFFFFFu, h.w), earlier = peers & ((1u << lane) - 1u);
+        const bool last = valid && (peers >> lane) == 1u;
+        const uint32_t pno = __popc(__ballot_sync(0xFFFFFFFFu, h.kind == LTPG_TPCC_NEWORDER) & earlier);
+        const uint32_t ppay = __popc(__ballot_sync(0xFFFFFFFFu, h.kind == LTPG_TPCC_PAYMENT) & earlier);
+        const uint32_t pdl = __popc(__ballot_sync(0xFFFFFFFFu, h.kind == LTPG_TPCC_DELIVERY) & earlier);
+        uint32_t pol = 0;  // h.cnt: lines of a NewOrder (at most 15), else 0
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) pol += __popc(__ballot_sync(0xFFFFFFFFu, (h.cnt >> i) & 1u) & earlier) << i;
         uint32_t bno = 0, bol = 0, bpay = 0, bdl = 0;
         if (valid) {
             bno = *ccp(a, CL_NO, h.w, g);
@@ -550,13 +573,43 @@ __global__ void __launch_bounds__(TB) tpcc_gen_rank(TpccGenArgs a) {
     }
 }
 
-// 5. NewOrder, Payment, StockLevel records.
+// 5. NewOrder, Payment, StockLevel records.  A block takes TB transactions,
+// NewOrders first, then the others, so that a warp draws one kind (a NewOrder
+// with its 5 to 15 lines takes ten times a Payment's draws); the items drawn so
+// far stand in shared memory for the check of a new one.  2^18 of the
+// five-transaction mix: 47 us in batch order, 34 us now.
 __global__ void __launch_bounds__(TB) tpcc_gen_main(TpccGenArgs a) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= a.B) return;
+    __shared__ uint32_t items[LTPG_TPCC_MAX_LINES][TB];
+    __shared__ uint16_t order[TB];
+    __shared__ uint32_t n_no[TB / 32], n_pay[TB / 32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, t0 = blockIdx.x * TB;
+    {
+        uint32_t kind = 0xFFFFFFFFu;
+        if (t0 + tid < a.B) {
+            Rng r = tpcc_rng(a, t0 + tid);
+            kind = tpcc_head(a.p, r).kind;
+        }
+        const bool no = kind == LTPG_TPCC_NEWORDER;
+        const bool pay = kind == LTPG_TPCC_PAYMENT || kind == LTPG_TPCC_STOCKLEVEL;
+        const unsigned bn = __ballot_sync(0xFFFFFFFFu, no), bp = __ballot_sync(0xFFFFFFFFu, pay);
+        if (lane == 0u) {
+            n_no[warp] = __popc(bn);
+            n_pay[warp] = __popc(bp);
+        }
+        order[tid] = 0xFFFFu;
+        __syncthreads();
+        uint32_t at = no ? __popc(bn & ((1u << lane) - 1u)) : __popc(bp & ((1u << lane) - 1u));
+        for (uint32_t i = 0; i < TB / 32; ++i) {
+            at += no ? (i < warp ? n_no[i] : 0u) : n_no[i];
+            if (pay && i < warp) at += n_pay[i];
+        }
+        if (no || pay) order[at] = (uint16_t)tid;
+        __syncthreads();
+    }
+    if (order[tid] == 0xFFFFu) return;
+    const uint32_t t = t0 + order[tid];
     Rng r = tpcc_rng(a, t);
     const TpccHead h = tpcc_head(a.p, r);
-    if (h.kind == LTPG_TPCC_ORDERSTATUS || h.kind == LTPG_TPCC_DELIVERY) return;
     ltpg_tpcc_txn x{};
     x.line_off = a.incl[t] - h.cnt;
     x.w = h.w;
@@ -565,7 +618,14 @@ __global__ void __launch_bounds__(TB) tpcc_gen_main(TpccGenArgs a) {
         x.a = (uint32_t)(((uint64_t)a.o_id[h.w] + s) % 30000u);
         x.b = (uint32_t)(((uint64_t)a.no_id[h.w] + s) % 30000u);
         x.c = (uint32_t)(((uint64_t)a.ol_id[h.w] + a.aux[t]) % 450000u);
-        tpcc_neworder(a.p, r, h, x, a.lines + x.line_off);
+        ltpg_tpcc_line *lines = a.lines + x.line_off;
+        tpcc_neworder(
+            a.p, r, h, x,
+            [&](uint32_t i, const ltpg_tpcc_line &ln) {
+                items[i][tid] = ln.i_id;
+                reinterpret_cast<uint2 *>(lines)[i] = make_uint2(ln.i_id, ln.supply_w | ((uint32_t)ln.qty << 16));
+            },
+            [&](uint32_t i) { return items[i][tid]; });
     } else if (h.kind == LTPG_TPCC_PAYMENT) {
         x.a = (uint32_t)(((uint64_t)a.h_id[h.w] + a.aux[t]) % 30000u);
         tpcc_payment(a.p, r, h, x, a.cust_name, a.cust_rank);
@@ -575,33 +635,45 @@ __global__ void __launch_bounds__(TB) tpcc_gen_main(TpccGenArgs a) {
     store_txn(a.txns + t, x);
 }
 
-// 6. Oldest undelivered order, per warehouse in batch order.  aux[t] of a
-// Delivery becomes DL_TRACKED | O_ID, or 0 when w had no undelivered order.
+// 6. Oldest undelivered order D, per warehouse in batch order: a Delivery that
+// follows M orders takes max(D, M - 30000) when D < M and leaves that + 1, which
+// with D <= M is min(max(D + 1, M - 29999), M).  Such steps compose to another
+// min(max(D + add, lo), hi), so a warp scans its warehouse's Deliveries 32 at a
+// time (one thread stepping through them: 40 us at W = 64 and 2^18 of the mix).
+// aux[t] of a Delivery becomes DL_TRACKED | O_ID, or 0 when w had no
+// undelivered order.
 __global__ void __launch_bounds__(TB) tpcc_gen_dl_walk(TpccGenArgs a) {
-    const uint32_t w = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
     if (w >= a.W) return;
-    uint64_t D = a.delivered[w];
-    const uint64_t M0 = a.made[w];
+    long long D = (long long)a.delivered[w];
+    const long long M0 = (long long)a.made[w];
     const uint32_t i1 = a.dl_start[w + 1];
-    for (uint32_t i = a.dl_start[w]; i < i1; i += 4) {
-        uint64_t e[4];
+    for (uint32_t i0 = a.dl_start[w]; i0 < i1; i0 += 32) {
+        const bool act = i0 + lane < i1;
+        const uint64_t e = act ? a.dl_list[i0 + lane] : 0ull;
+        const long long M = M0 + (long long)(e >> 32);
+        // this lane's step, then the steps of lanes 0 .. lane composed; a lane
+        // past the end adds nothing
+        long long add = act ? 1 : 0, lo = act ? M - 29999 : -(1ll << 60), hi = act ? M : 1ll << 60;
 #pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) e[j] = i + j < i1 ? a.dl_list[i + j] : 0ull;
-#pragma unroll
-        for (uint32_t j = 0; j < 4; ++j) {
-            if (i + j >= i1) break;
-            const uint32_t t = (uint32_t)e[j];
-            const uint64_t M = M0 + (e[j] >> 32);
-            uint32_t v = 0;
-            if (D < M) {
-                if (M - D > 30000u) D = M - 30000u;
-                v = DL_TRACKED | (uint32_t)(D % 30000u);
-                ++D;
+        for (uint32_t o = 1; o < 32; o <<= 1) {
+            const long long add0 = __shfl_up_sync(0xFFFFFFFFu, add, o), lo0 = __shfl_up_sync(0xFFFFFFFFu, lo, o),
+                            hi0 = __shfl_up_sync(0xFFFFFFFFu, hi, o);
+            if (lane >= o) {
+                const long long l = min(max(lo0 + add, lo), hi), u = min(max(hi0 + add, lo), hi);
+                add += add0;
+                lo = l;
+                hi = u;
             }
-            a.aux[t] = v;
         }
+        const long long after = min(max(D + add, lo), hi);
+        long long before = __shfl_up_sync(0xFFFFFFFFu, after, 1);
+        if (lane == 0u) before = D;
+        if (act)
+            a.aux[(uint32_t)e] = before < M ? DL_TRACKED | (uint32_t)((uint64_t)max(before, M - 30000) % 30000u) : 0u;
+        D = __shfl_sync(0xFFFFFFFFu, after, 31);
     }
-    a.delivered[w] = D;
+    if (lane == 0u) a.delivered[w] = (uint64_t)D;
 }
 
 // 7. OrderStatus and Delivery records.
@@ -723,7 +795,7 @@ cudaError_t bind_tpcc(ltpg_gen *g, int device) {
     if (!d) return cudaErrorMemoryAllocation;
     d->device = device;
     const uint32_t B = g->c.n_txn, W = g->c.warehouses;
-    d->C = 1024;
+    d->C = 128;
     if ((uint64_t)((B + d->C - 1) / d->C) * W > MAX_CHUNK_COUNTERS) {
         const uint64_t g_max = std::max<uint64_t>(1, MAX_CHUNK_COUNTERS / W);
         d->C = (uint32_t)(((B + g_max - 1) / g_max + 31) / 32 * 32);
@@ -910,13 +982,13 @@ int gen_tpcc(ltpg_ctx *c, ltpg_gen *g, uint64_t batch_id, uint32_t slot, cudaStr
     }
     if (e == cudaSuccess) e = inclusive_scan(a.incl, a.B, d->blk, st, launches);
     if (e == cudaSuccess) {
-        tpcc_gen_chunk_scan<<<blocks(4ull * a.W * 32, TB), TB, 0, st>>>(a);
+        tpcc_gen_chunk_scan<<<4u * a.W, TB, 0, st>>>(a);
         tpcc_gen_starts<<<1, SCAN_T, 0, st>>>(a);
         tpcc_gen_rank<<<blocks((uint64_t)a.G * 32, TB), TB, 0, st>>>(a);
         tpcc_gen_main<<<nb, TB, 0, st>>>(a);
         launches += 4;
         if (a.tracking) {
-            tpcc_gen_dl_walk<<<blocks(a.W, TB), TB, 0, st>>>(a);
+            tpcc_gen_dl_walk<<<blocks(32ull * a.W, TB), TB, 0, st>>>(a);
             ++launches;
         }
         tpcc_gen_osdl<<<nb, TB, 0, st>>>(a);
