@@ -400,8 +400,8 @@ int ltpg_commit_bitmap_device(ltpg_ctx *ctx, uint32_t slot, const uint32_t **dev
  * a later batch).  It saves the row reads of aborted transactions. */
 typedef struct {
     uint32_t block_threads;   /* threads per block of the tuned kernels: 128, 256
-                                 or 512 (TPC-C: tiles of 64, 128 or 256
-                                 transactions)                                  */
+                                 or 512 (TPC-C: on tiles of up to as
+                                 many transactions)                             */
     uint32_t ops_per_thread;  /* YCSB op words per thread: 1, 2, 4 or 8         */
     uint32_t blocks_per_sm;   /* cap on resident blocks per SM, 0 = occupancy   */
     uint32_t stage_ways;      /* shared-memory staging entries per hot bucket   */

@@ -141,7 +141,7 @@ int epoch_reserve(ltpg_ctx *c, uint64_t batches) {
     if (c->ycsb.reg)
         CK(cudaMemsetAsync(c->ycsb.reg, 0xFF, c->ycsb.n * sizeof(RegSlot), c->stream), "clear YCSB slots");
     if (c->tpcc.reg)
-        CK(cudaMemsetAsync(c->tpcc.reg, 0xFF, c->tpcc.n_slots * sizeof(RegSlot), c->stream), "clear TPC-C slots");
+        CK(tpcc_clear_slots(c), "clear TPC-C slots");
     CK(ctl_set_epoch(c->ctl, 1u, c->stream), "reset epoch");
     c->epoch_next = 1 + batches;
     return LTPG_OK;
@@ -208,6 +208,9 @@ int ltpg_destroy(ltpg_ctx *c) {
     for (auto &t : c->tpcc.tab) dev_free(t);
     dev_free(c->tpcc.reg);
     dev_free(c->tpcc.name_idx);
+    dev_free(c->tpcc.name_dir);
+    dev_free(c->tpcc.claim);
+    dev_free(c->tpcc.stock_w);
     dev_free(c->stage_map);
     dev_free(c->stage_bits);
     dev_free(c->stage_rank);
@@ -272,6 +275,9 @@ int ltpg_db_load_tpcc(ltpg_ctx *c, uint64_t seed, uint32_t W) {
     for (auto &t : c->tpcc.tab) dev_free(t);
     dev_free(c->tpcc.reg);
     dev_free(c->tpcc.name_idx);
+    dev_free(c->tpcc.name_dir);
+    dev_free(c->tpcc.claim);
+    dev_free(c->tpcc.stock_w);
     c->tpcc = TpccDb{};
     uint64_t total = 0;
     for (uint32_t t = 0; t < LTPG_TPCC_TABLES; ++t) {
@@ -283,6 +289,9 @@ int ltpg_db_load_tpcc(ltpg_ctx *c, uint64_t seed, uint32_t W) {
     if (total >= (1ull << 32)) return fail(c, LTPG_ERR_INVALID, "too many rows for 32-bit slots");
     CK(dev_alloc(&c->tpcc.reg, total), "alloc TPC-C registration table");
     CK(dev_alloc(&c->tpcc.name_idx, c->tpcc.rows[LTPG_T_CUSTOMER]), "alloc customer name index");
+    CK(dev_alloc(&c->tpcc.name_dir, 10ull * W * NAME_DIR_LEN), "alloc customer name directory");
+    CK(dev_alloc(&c->tpcc.claim, claim_total_words(W)), "alloc claim bitmaps");
+    CK(dev_alloc(&c->tpcc.stock_w, c->tpcc.rows[LTPG_T_STOCK]), "alloc stock writers");
     c->tpcc.n_slots = total;
     c->tpcc.W = W;
     c->tpcc_seed = seed;
@@ -389,7 +398,8 @@ int slot_prepare_ycsb(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint32_t k, ui
     return LTPG_OK;
 }
 
-int slot_prepare_tpcc(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint64_t n_lines, uint64_t txn_base, Slot **out) {
+int slot_prepare_tpcc(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint64_t n_lines, uint64_t txn_base,
+                      bool reads_orders, Slot **out) {
     Slot *s = get_slot(c, slot);
     if (!s) return fail(c, LTPG_ERR_INVALID, "bad slot or batch");
     if (!c->tpcc.W) return fail(c, LTPG_ERR_STATE, "no TPC-C tables loaded");
@@ -404,8 +414,9 @@ int slot_prepare_tpcc(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint64_t n_lin
     }
     int r = ensure_outputs(c, *s, n_txn);
     if (r) return r;
-    if (s->workload != LTPG_WORKLOAD_TPCC || s->n_txn != n_txn) drop_graphs(c);
+    if (s->workload != LTPG_WORKLOAD_TPCC || s->n_txn != n_txn || s->reads_orders != reads_orders) drop_graphs(c);
     s->workload = LTPG_WORKLOAD_TPCC;
+    s->reads_orders = reads_orders;
     s->n_txn = n_txn;
     s->n_lines = (uint32_t)n_lines;
     s->txn_base = txn_base;
@@ -449,7 +460,13 @@ int upload_tpcc(ltpg_ctx *c, uint32_t slot, const ltpg_tpcc_batch *b, cudaStream
     if (!c || !b) return c ? fail(c, LTPG_ERR_INVALID, "bad slot or batch") : LTPG_ERR_INVALID;
     if (!b->txns || (b->n_lines && !b->lines && !packed)) return fail(c, LTPG_ERR_INVALID, "null batch array");
     Slot *s = nullptr;
-    int r = slot_prepare_tpcc(c, slot, b->n_txn, b->n_lines, b->txn_base, &s);
+    // 64 records spread over the batch tell a mix with OrderStatus or Delivery
+    bool reads_orders = false;
+    for (uint32_t i = 0; i < 64u && b->n_txn >= CLAIM_MIN_TXNS; ++i) {
+        const uint32_t kind = tpcc_kind(b->txns[(uint64_t)b->n_txn * i / 64u].kind_info);
+        reads_orders |= kind == LTPG_TPCC_ORDERSTATUS || kind == LTPG_TPCC_DELIVERY;
+    }
+    int r = slot_prepare_tpcc(c, slot, b->n_txn, b->n_lines, b->txn_base, reads_orders, &s);
     if (r) return r;
     CK(cudaMemcpyAsync(s->txns, b->txns, (uint64_t)b->n_txn * sizeof(ltpg_tpcc_txn), cudaMemcpyHostToDevice, st),
        "upload txns");

@@ -73,10 +73,23 @@ struct TpccDb {
     uint64_t n_slots = 0;
     RegSlot *reg = nullptr;  // flat over all tables
     uint64_t base[LTPG_TPCC_TABLES] = {};
+    // Claims of a batch (tuned path): bitmaps of claim_total_words() words, and
+    // the STOCK rows' smallest writers, epoch-tagged like a slot's.
+    uint32_t *claim = nullptr;
+    unsigned long long *stock_w = nullptr;
     // Customer last-name index: per district its 3,000 keys
     // (min(C_LAST, 2^32 - 1) << 32 | C_ID) in ascending order.
     uint64_t *name_idx = nullptr;
+    // and per district the first index position of each name below NAME_DIR
+    uint16_t *name_dir = nullptr;
 };
+constexpr uint32_t NAME_DIR = 1024, NAME_DIR_LEN = NAME_DIR + 1;
+
+// Words of one bitmap over HISTORY, NEW-ORDER, ORDER and ORDER-LINE (540,000
+// rows a warehouse), and of a batch's claims: two of them, two flags, and a
+// bitmap over STOCK.
+inline uint32_t claim_words(uint32_t W) { return (uint32_t)((540000ull * W + 31) / 32); }
+inline uint64_t claim_total_words(uint32_t W) { return 2ull * claim_words(W) + 2 + 3125ull * W; }
 
 // One device batch slot.
 struct Slot {
@@ -92,6 +105,10 @@ struct Slot {
     // TPC-C
     uint32_t n_lines = 0;
     uint64_t txn_base = 0;
+    // A batch of CLAIM_MIN_TXNS or more has OrderStatus or Delivery transactions
+    // (a device-made batch's mix; a sample of an uploaded one's): says which
+    // registration is likely faster, both give the same outcome.
+    bool reads_orders = false;
     ltpg_tpcc_txn *txns = nullptr;
     ltpg_tpcc_line *lines = nullptr;
     uint32_t *packed_lines = nullptr;  // packed uploads land here before their unpacking
@@ -185,7 +202,9 @@ void drop_graphs_ctx(ltpg_ctx *c);
 // Readies slot `slot` for a batch of the given shape (buffers, outputs, graph
 // invalidation) and records the shape; the caller fills the batch buffers.
 int slot_prepare_ycsb(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint32_t k, uint32_t n_updates, Slot **out);
-int slot_prepare_tpcc(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint64_t n_lines, uint64_t txn_base, Slot **out);
+constexpr uint32_t CLAIM_MIN_TXNS = 131072;  // tpcc.cu, tpcc_claims
+int slot_prepare_tpcc(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint64_t n_lines, uint64_t txn_base,
+                      bool reads_orders, Slot **out);
 // Makes generator g's batch batch_id in slot `slot` on stream st (gen_dev.cu).
 int gen_device_batch(ltpg_ctx *c, ltpg_gen *g, uint64_t batch_id, uint32_t slot, cudaStream_t st);
 // Makes room for `batches` more batch epochs before a launch (resets the
@@ -210,6 +229,8 @@ cudaError_t ycsb_derive_offsets(ltpg_ctx *c, Slot &s, cudaStream_t st);
 cudaError_t tpcc_unpack_lines(Slot &s, cudaStream_t st);
 cudaError_t ycsb_run_tuned(ltpg_ctx *c, Slot &s, int mode);   // fused / persistent
 cudaError_t tpcc_init_tables(ltpg_ctx *c);
+// Every TPC-C registration slot back to the cleared state, on the context stream.
+cudaError_t tpcc_clear_slots(ltpg_ctx *c);
 cudaError_t tpcc_build_name_index(ltpg_ctx *c);
 cudaError_t tpcc_phase(ltpg_ctx *c, Slot &s, int phase);
 cudaError_t tpcc_run_tuned(ltpg_ctx *c, Slot &s, int mode);

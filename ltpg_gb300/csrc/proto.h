@@ -138,21 +138,6 @@ LTPG_HD uint32_t tpcc_n_ops(uint32_t kind_info) {
     default: return 1u;
     }
 }
-// Ops that can conflict, apart from order lines (the tuned kernels' header
-// ops): reads of WAREHOUSE, DISTRICT and ITEM rows never can (no transaction
-// registers a write there), so NewOrder and Payment keep ops j = 2, 3, 4 and
-// the other kinds all of theirs.
-LTPG_HD uint32_t tpcc_n_head(uint32_t kind_info) {
-    switch (tpcc_kind(kind_info)) {
-    case LTPG_TPCC_DELIVERY: return 4u;
-    case LTPG_TPCC_STOCKLEVEL: return 1u;
-    default: return 3u;
-    }
-}
-LTPG_HD uint32_t tpcc_head_j(uint32_t kind_info, uint32_t k) {
-    const uint32_t kind = tpcc_kind(kind_info);
-    return (kind == LTPG_TPCC_NEWORDER || kind == LTPG_TPCC_PAYMENT) ? k + 2u : k;
-}
 LTPG_HD bool tpcc_customer_by_name(uint32_t kind_info) {
     const uint32_t kind = tpcc_kind(kind_info);
     return (kind == LTPG_TPCC_PAYMENT || kind == LTPG_TPCC_ORDERSTATUS) && (kind_info & LTPG_PAY_BY_NAME);
