@@ -49,7 +49,7 @@ struct YcsbTunedArgs {
     uint32_t *bucket_counts;
     uint32_t ways, stage_entries;
     uint32_t filter;
-    uint32_t lpt;  // lanes per transaction of the one-op-per-lane kernels: stride rounded up to a power of two (0: > 32)
+    uint32_t lpt;  // lanes per transaction of the one-op-per-lane kernels: stride (at most 32) rounded up to a power of two
     uint32_t late; // late reads: 0 off, 1 in the check kernel's tiles, 2 in a kernel of their own,
                    // 3 write-first registration
     uint32_t *wbits;  // write-first: one bit per key, set for keys an update of the batch writes
@@ -87,84 +87,6 @@ __device__ __forceinline__ uint32_t ld_wbits(const uint32_t *p) {
 template <bool kCoh>
 __device__ __forceinline__ uint32_t ld_flag(const uint8_t *p) {
     return kCoh ? ld_gpu_u8(p) : (uint32_t)*p;
-}
-
-// ---- execute + register over all tiles assigned to this block ----------------
-template <bool kStage>
-__device__ __forceinline__ void exec_tiles(const YcsbTunedArgs &a, unsigned long long *dig, StageEnt *tab,
-                                           uint64_t tag) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t nvec_tile = a.tile * a.stride / 4;
-    const uint32_t n_tiles = (a.B + a.tile - 1) / a.tile;
-    uint32_t counted = 0;
-    for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-        const uint32_t t0 = tile * a.tile;
-        const uint32_t nt = min(a.tile, a.B - t0);
-        const uint32_t nvec = nt * a.stride / 4;
-        for (uint32_t i = threadIdx.x; i < a.tile; i += blockDim.x) dig[i] = 0ull;
-        __syncthreads();
-        const uint4 *vp = reinterpret_cast<const uint4 *>(a.ops + (uint64_t)t0 * a.stride);
-        for (uint32_t base = 0; base < nvec_tile; base += blockDim.x) {
-            const uint32_t v = base + threadIdx.x;
-            const bool act = v < nvec;
-            const uint4 w4 = act ? ld_nc_u4(vp + v) : make_uint4(LTPG_YCSB_OP_PAD, LTPG_YCSB_OP_PAD,
-                                                                  LTPG_YCSB_OP_PAD, LTPG_YCSB_OP_PAD);
-            const uint32_t lt = act ? (v * 4) / a.stride : 0;
-            const uint32_t j0 = v * 4 - lt * a.stride;
-            const uint32_t t = t0 + lt;
-            const uint32_t words[4] = {w4.x, w4.y, w4.z, w4.w};
-            unsigned long long part = 0;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const uint32_t w = words[q];
-                bool valid = act && !ycsb_is_pad(w);
-                const uint32_t key = ycsb_key(w);
-                const bool upd = ycsb_is_update(w);
-                if (valid && key >= a.n) {
-                    report_error(a.ctl, DERR_BOUNDS, t);
-                    valid = false;
-                }
-                bool staged = false;
-                if (kStage && valid) {
-                    const uint32_t b = key_bucket(key);
-                    const uint32_t g = __ldg(a.stage_map + b);
-                    if (g != STAGE_NONE && (g + 1) * a.ways <= a.stage_entries) {
-                        StageEnt *e = stage_find(tab, g, a.ways, key);
-                        if (e) {
-                            atomicMin(upd ? &e->wmin : &e->rmin, t);
-                            atomicAdd(&e->cnt, 1u);
-                            staged = true;
-                        }
-                    }
-                    if (!staged && (t % COUNT_SAMPLE) == 0u) {
-                        atomicAdd(a.bucket_counts + b, COUNT_SAMPLE);
-                        ++counted;
-                    }
-                }
-                const bool need = valid && !staged;
-                const uint32_t mkey = need ? (key | (upd ? 0x80000000u : 0u)) : 0xFFFFFFFFu;
-                const unsigned peers = __match_any_sync(FULL, mkey);
-                // lanes are in transaction order, so the lowest peer holds the smallest TID
-                if (need && (__ffs(peers) - 1) == (int)lane) {
-                    unsigned long long *slot = upd ? &a.reg[key].w : &a.reg[key].r;
-                    const unsigned long long mine = tag | t;
-                    if (!a.filter || ld_ca_u64(slot) > mine) red_min(slot, mine);
-                }
-                if (valid && !upd) {
-                    const char *p = reinterpret_cast<const char *>(a.rows + (uint64_t)key * LTPG_YCSB_FIELDS);
-                    const ulonglong2 r0 = ld_nc16(p), r1 = ld_nc16(p + 16), r2 = ld_nc16(p + 32),
-                                     r3 = ld_nc16(p + 48), r4 = ld_nc16(p + 64);
-                    const unsigned long long x = r0.x ^ r0.y ^ r1.x ^ r1.y ^ r2.x ^ r2.y ^ r3.x ^ r3.y ^ r4.x ^ r4.y ^
-                                                 scan_rest(a.reg, a.rows, a.n, w, tag | t, a.filter != 0u);
-                    part += x * (2ull * (j0 + q) + 1ull);
-                }
-            }
-            if (part) atomicAdd(&dig[lt], part);
-        }
-        __syncthreads();
-        for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) a.results[t0 + i] = (int64_t)dig[i];
-    }
-    (void)counted;
 }
 
 // Stores the updates of committed transaction t in op order: a transaction
@@ -639,47 +561,92 @@ __device__ __forceinline__ void wf_check_list(const YcsbTunedArgs &a, uint32_t e
 template <int BS>
 __global__ void __launch_bounds__(BS) ycsb_wf_check_list(YcsbTunedArgs a) { wf_check_list<false>(a, a.ctl->epoch); }
 
+// Shared memory layout: [off: tile + 1 u32][fl: tile u32][upd: tile * stride / 4
+// bytes, the updates of each op vector][stage table]; a tile is a multiple of 32.
+__host__ __device__ __forceinline__ size_t ycsb_smem_bytes(uint32_t tile, uint32_t stride, uint32_t stage_entries) {
+    return (size_t)tile * 8 + 16 + (size_t)tile * (stride / 4u) + (size_t)stage_entries * sizeof(StageEnt);
+}
+
+struct SmemPtrs {
+    uint32_t *off, *fl;
+    uint8_t *upd;
+    StageEnt *tab;
+};
+__device__ __forceinline__ SmemPtrs carve(char *base, uint32_t tile, uint32_t stride) {
+    SmemPtrs p;
+    p.off = reinterpret_cast<uint32_t *>(base);
+    p.fl = reinterpret_cast<uint32_t *>(base + (size_t)tile * 4 + 16);
+    p.upd = reinterpret_cast<uint8_t *>(p.fl + tile);
+    p.tab = reinterpret_cast<StageEnt *>(base + ycsb_smem_bytes(tile, stride, 0));
+    return p;
+}
+
 // ---- check + write-back over all tiles assigned to this block ------------------
-// fl: tile flags.  kLate = 0: the third pass stores the committed updates;
-// 1: it reads the committed transactions' rows (late_read_tile); 2: there is
-// no third pass (the reads have a kernel of their own).  With late reads the
-// updates are stored by a later kernel.
+// fl: tile flags; off: the tile's value offsets.  kLate = 0: the third pass
+// stores the committed updates; 1: it reads the committed transactions' rows
+// (late_read_tile); 2: there is no third pass (the reads have a kernel of their
+// own).  With late reads the updates are stored by a later kernel.
+// Each pass is a chain of dependent loads, which bounds a batch of one wave, so
+// a thread issues two slot loads together, the value offsets are on their way
+// during the check, and an update is stored by the thread that holds its op
+// word (one thread per transaction took its vectors in turn).  Slots come
+// through L1: a hot key's is loaded by every warp, and its L2 slice was the
+// bound at high skew.  In the persistent kernel the grid barrier's fences order
+// these loads behind the registrations.  (65,536 x 10, half updates: theta 0.6
+// 17 -> 12.4 us, 0.99 25 -> 11 us; 2^18 x 10 of 10 M at 0.99: 79 -> 33 us;
+// 2,000 x 10: 10 -> 8.3 us.)
+__device__ __forceinline__ ulonglong2 ld_slot_if(bool on, const RegSlot *p) {
+    ulonglong2 v = make_ulonglong2(~0ull, ~0ull);  // nobody's
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %3, 0; @q ld.global.ca.v2.u64 {%0, %1}, [%2]; }"
+                 : "+l"(v.x), "+l"(v.y) : "l"(p), "r"((uint32_t)on));
+    return v;
+}
+
 template <int kLate>
-__device__ __forceinline__ void checkwb_tiles(const YcsbTunedArgs &a, uint32_t *fl, RowScratch *ws, uint32_t epoch) {
+__device__ __forceinline__ void checkwb_tiles(const YcsbTunedArgs &a, const SmemPtrs &sm, RowScratch *ws,
+                                              uint32_t epoch) {
+    uint32_t *fl = sm.fl, *off = sm.off;
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t nvec_tile = a.tile * a.stride / 4;
+    const uint32_t vpt = a.stride / 4;  // vectors of a transaction
     const uint32_t n_tiles = (a.B + a.tile - 1) / a.tile;
+    const uint64_t nv = kLate ? 0ull : min((uint64_t)__ldg(a.val_off + a.B), a.vals_cap);
     TxnCounts cnt;
     for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
         const uint32_t t0 = tile * a.tile;
         const uint32_t nt = min(a.tile, a.B - t0);
-        const uint32_t nvec = nt * a.stride / 4;
-        for (uint32_t i = threadIdx.x; i < a.tile; i += blockDim.x) fl[i] = 0u;
-        __syncthreads();
+        const uint32_t nvec = nt * vpt;
         const uint4 *vp = reinterpret_cast<const uint4 *>(a.ops + (uint64_t)t0 * a.stride);
+        uint4 w4 = make_uint4(0u, 0u, 0u, 0u);
+        if (threadIdx.x < nvec) w4 = ld_nc_u4(vp + threadIdx.x);
+        for (uint32_t i = threadIdx.x; i < a.tile; i += blockDim.x) fl[i] = 0u;
+        if (!kLate)
+            for (uint32_t i = threadIdx.x; i <= nt; i += blockDim.x) off[i] = __ldg(a.val_off + t0 + i);
+        __syncthreads();
         // pass 1: conflict flags per transaction
-        for (uint32_t base = 0; base < nvec_tile; base += blockDim.x) {
-            const uint32_t v = base + threadIdx.x;
-            if (v >= nvec) continue;
-            const uint4 w4 = ld_nc_u4(vp + v);
-            const uint32_t lt = (v * 4) / a.stride;
-            const uint32_t t = t0 + lt;
+        for (uint32_t v = threadIdx.x; v < nvec; v += blockDim.x) {
+            const uint32_t lt = v / vpt, t = t0 + lt;
+            if (v >= blockDim.x) w4 = ld_nc_u4(vp + v);
             const uint32_t words[4] = {w4.x, w4.y, w4.z, w4.w};
             uint32_t f = 0;
+            ulonglong2 s[2];  // two slots in flight: four take the registers of a block
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
+                if (q % 2 == 0)
+#pragma unroll
+                    for (int r = 0; r < 2; ++r)
+                        s[r] = ld_slot_if(!ycsb_is_pad(words[q + r]) && ycsb_key(words[q + r]) < a.n,
+                                          a.reg + ycsb_key(words[q + r]));
                 const uint32_t w = words[q];
-                if (ycsb_is_pad(w) || ycsb_key(w) >= a.n) continue;
-                const ulonglong2 s = ld_slot(a.reg + ycsb_key(w));
-                const uint32_t rmin = slot_min(s.x, epoch), wmin = slot_min(s.y, epoch);
+                const uint32_t rmin = slot_min(s[q % 2].x, epoch), wmin = slot_min(s[q % 2].y, epoch);
                 if (ycsb_is_update(w)) {
                     if (rmin < t) f |= LTPG_FLAG_WAR;
                     if (wmin < t) f |= LTPG_FLAG_WAW;
-                } else if (wmin < t || scan_rest_raw(a.reg, a.n, w, t, epoch)) {
+                } else if (wmin < t || (!ycsb_is_pad(w) && ycsb_key(w) < a.n && scan_rest_raw(a.reg, a.n, w, t, epoch))) {
                     f |= LTPG_FLAG_RAW;
                 }
             }
             if (f) atomicOr(&fl[lt], f);
+            if (!kLate) sm.upd[v] = (uint8_t)vec_updates(words);
         }
         __syncthreads();
         // pass 2: commit decision, flags, bitmap words (tile is a multiple of 32)
@@ -704,13 +671,46 @@ __device__ __forceinline__ void checkwb_tiles(const YcsbTunedArgs &a, uint32_t *
             }
         }
         __syncthreads();
-        // pass 3: committed updates, one thread per transaction in op order
-        // (or, with late reads, the committed transactions' row reads)
+        // pass 3: committed updates (or, with late reads, the committed
+        // transactions' row reads)
         if (kLate == 1) {
             late_read_tile(a, ws, fl, t0, nt);
         } else if (kLate == 0) {
-            for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x)
-                if (fl[i] & LTPG_FLAG_COMMIT) write_txn_updates(a, t0 + i);
+            // A transaction that updates a field twice leaves its later value, as
+            // a sequential replay does: its vectors store one after another,
+            // a barrier apart.  No two committed transactions write one row (WAW).
+            for (uint32_t base = 0; base < nvec; base += blockDim.x) {
+                const uint32_t v = base + threadIdx.x, lt = v / vpt, at = v - lt * vpt;
+                uint64_t *to[4];
+                uint64_t val[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) to[q] = nullptr;
+                if (v < nvec && sm.upd[v] && (fl[lt] & LTPG_FLAG_COMMIT) && off[lt] != off[lt + 1]) {
+                    uint64_t idx = off[lt];
+                    for (uint32_t u = 1; u <= at; ++u) idx += sm.upd[v - u];
+                    w4 = ld_nc_u4(vp + v);
+                    const uint32_t words[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const uint32_t w = words[q], key = ycsb_key(w), fld = ycsb_field(w);
+                        if (ycsb_is_pad(w) || !ycsb_is_update(w)) continue;
+                        if (idx >= nv) {  // offsets that disagree with the op words
+                            report_error(a.ctl, DERR_BOUNDS, t0 + lt);
+                        } else if (key < a.n && fld < LTPG_YCSB_FIELDS) {
+                            to[q] = a.rows + (uint64_t)key * LTPG_YCSB_FIELDS + fld;
+                            val[q] = __ldg(a.vals + idx);
+                        }
+                        ++idx;
+                    }
+                }
+                for (uint32_t s = 0; s < vpt; ++s) {
+                    if (s) __syncthreads();
+                    if (s == at)
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            if (to[q]) *to[q] = val[q];
+                }
+            }
         }
         __syncthreads();
     }
@@ -852,23 +852,60 @@ __global__ void __launch_bounds__(BS) ycsb_exec_fast(YcsbTunedArgs a, uint32_t l
 // handed back to the lane that owns the op.
 // kReads = false (late reads): registration only; the rows are read after the
 // check, by the committed transactions alone (late_read_tile).
-template <bool kStage, bool kFilter, bool kDedupe, bool kReads>
+// kDedupe: one registration per distinct (key, kind), of a warp by match_any
+// (DEDUPE_WARP) or of the block (DEDUPE_BLOCK), by the first thread with it,
+// which holds the smallest TID.  For a block: a bucket of a table in shared
+// memory ends up with the step's smallest entry: step number (counting down, so
+// that nothing is cleared between steps), the rest of the mixed key, thread.  A
+// thread that finds a smaller thread of its own key there leaves the
+// registration to it; one that finds anything else (another key, a later
+// step's entry: the barrier is once a step) sends.  And all but the first
+// eighth of the lanes send after their row reads, past a look at the slot,
+// which by then holds the TIDs of that eighth if the key is hot.
+// Reductions on neighbouring hot slots queue at one slice of L2, and in a batch
+// of one wave no slot has been written when it is first looked at (10,000 x 10,
+// theta 0.99: 18 us with one lane's registration per warp, 13.4 with the table,
+// 8.4 with the late look).
+enum : int { DEDUPE_NONE, DEDUPE_WARP, DEDUPE_BLOCK };
+constexpr uint32_t OP_KEY_BITS = LTPG_YCSB_KEY_BITS + 1;  // key and kind
+template <int BS>
+__device__ __forceinline__ uint32_t *op_table() {
+    __shared__ uint32_t t[4 * BS];
+    return t;
+}
+
+template <bool kStage, bool kFilter, int kDedupe, bool kReads, int BS>
 __device__ __forceinline__ void coop_exec_loop(const YcsbTunedArgs &a, StageEnt *tab, const uint32_t *sbits,
                                                const uint32_t *srank, RowScratch *ws,
                                                uint64_t tag) {
+    constexpr bool kTable = kDedupe == DEDUPE_BLOCK, kPeers = kDedupe == DEDUPE_WARP || kStage;
+    constexpr uint32_t kBits = BS == 128 ? 9 : BS == 256 ? 10 : 11, kRest = OP_KEY_BITS - kBits;  // 4 BS buckets
+    constexpr uint32_t kSteps = 1u << (32 - 9 - kRest);
+    static_assert(BS <= 512 && kRest + 9 < 32, "an entry is step | rest | thread");
+    uint32_t *ops_tab = nullptr;
+    uint32_t steps = 0;  // left before the table is cleared
+    if (kTable) ops_tab = op_table<BS>();
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t lpt = a.lpt;  // lanes per transaction, a power of two
     const uint32_t lsh = (uint32_t)__ffs(lpt) - 1u;
     const uint32_t groups = a.ways ? a.stage_entries / a.ways : 0u;
     const uint64_t nw = (uint64_t)a.B << lsh;
     const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+    // lanes that register before their row reads: all where no filter is asked
+    // for and the batch takes more than two steps
+    const uint64_t early = kFilter || nw <= 2u * step ? step / 8u : ~0ull;
     bool scans = false;  // some read of this thread's was a range scan
+    const uint32_t j = threadIdx.x & (lpt - 1u);  // blocks start at whole transactions
+    auto op_at = [&](uint64_t v) {
+        return v < nw && j < a.stride ? __ldg(a.ops + (v >> lsh) * a.stride + j) : LTPG_YCSB_OP_PAD;
+    };
+    uint32_t next = op_at((uint64_t)blockIdx.x * blockDim.x + threadIdx.x);  // one step ahead of its use
     for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < nw; base += step) {
         const uint64_t v = base + threadIdx.x;
         const bool act = v < nw;
         const uint32_t t = (uint32_t)(v >> lsh);
-        const uint32_t j = (uint32_t)v & (lpt - 1u);
-        const uint32_t w = act && j < a.stride ? __ldg(a.ops + (uint64_t)t * a.stride + j) : LTPG_YCSB_OP_PAD;
+        const uint32_t w = next;
+        next = op_at(v + step);
         bool valid = act && !ycsb_is_pad(w);
         const uint32_t key = ycsb_key(w);
         if (valid && key >= a.n) {
@@ -891,9 +928,23 @@ __device__ __forceinline__ void coop_exec_loop(const YcsbTunedArgs &a, StageEnt 
                 have_dig = true;
             }
         }
+        uint32_t entry = 0, bucket = 0;
+        if (kTable) {
+            if (steps == 0u) {
+                __syncthreads();
+                for (uint32_t i = threadIdx.x; i < 4u * BS; i += blockDim.x) ops_tab[i] = ~0u;
+                __syncthreads();
+                steps = kSteps - 1u;  // the largest stays for the cleared state
+            }
+            --steps;
+            const uint32_t h = ((key | (upd ? 1u << LTPG_YCSB_KEY_BITS : 0u)) * 0x9E3779B1u) & ((1u << OP_KEY_BITS) - 1u);
+            bucket = h >> kRest;
+            entry = (((steps << kRest) | (h & ((1u << kRest) - 1u))) << 9) | threadIdx.x;
+            if (valid) atomicMin(ops_tab + bucket, entry);
+        }
         // one row read per distinct key of the warp: peers share the leader's
         unsigned peers = 1u << lane;
-        if (kDedupe || kStage) peers = __match_any_sync(FULL, valid ? (key | (upd ? 0x80000000u : 0u)) : 0xFFFFFFFFu);
+        if (kPeers) peers = __match_any_sync(FULL, valid ? (key | (upd ? 0x80000000u : 0u)) : 0xFFFFFFFFu);
         const uint32_t leader_lane = (uint32_t)__ffs(peers) - 1u;
         const bool leader = valid && leader_lane == lane;
         // rows still to read
@@ -906,20 +957,28 @@ __device__ __forceinline__ void coop_exec_loop(const YcsbTunedArgs &a, StageEnt 
         const bool need_global = valid && !e;
         uint64_t cur = ~0ull;
         unsigned long long *slot = upd ? &a.reg[key].w : &a.reg[key].r;
-        if (kFilter && need_global) cur = ld_ca_u64(slot);
+        if (kFilter && !kTable && need_global) cur = ld_ca_u64(slot);
         if (kStage && e && leader) {
             atomicMin(upd ? &e->wmin : &e->rmin, t);
             atomicAdd(&e->cnt, (uint32_t)__popc(peers));
         }
         const unsigned long long mine = tag | t;
-        if (need_global && (kDedupe ? leader : true) && cur > mine) red_min_exec(slot, mine);
+        bool send = need_global && (leader || kDedupe == DEDUPE_NONE);
+        if (kTable) {
+            __syncthreads();
+            const uint32_t best = ops_tab[bucket];
+            send = need_global && (best == entry || ((best ^ entry) >> 9) != 0u);
+        }
+        const bool late = kTable && base >= early;
+        if (send && !late && cur > mine) red_min_exec(slot, mine);
         scans |= rd && ycsb_span(w) != 0u;
-        if (!kReads) continue;
-        if (need) {
+        if (kReads && need) {
             const unsigned long long rowx = kStage ? rows_fold_shfl(need, ch) : rows_fold(ws, need, ch);
             if ((need >> lane) & 1u) x = rowx;
         }
-        if (kDedupe || kStage) {
+        if (send && late && ld_ca_u64(slot) > mine) red_min_exec(slot, mine);
+        if (!kReads) continue;
+        if (kPeers) {
             const unsigned long long from_leader = __shfl_sync(FULL, x, leader_lane);
             if (!have_dig) x = from_leader;
         }
@@ -988,7 +1047,7 @@ __device__ __forceinline__ void coop_exec_loop(const YcsbTunedArgs &a, StageEnt 
     }
 }
 
-template <bool kStage, bool kFilter, bool kDedupe, bool kReads, int BS>
+template <bool kStage, bool kFilter, int kDedupe, bool kReads, int BS>
 __global__ void __launch_bounds__(BS) ycsb_exec_coop(YcsbTunedArgs a) {
     extern __shared__ __align__(16) char smem[];
     uint32_t *sbits = reinterpret_cast<uint32_t *>(smem);
@@ -1003,7 +1062,7 @@ __global__ void __launch_bounds__(BS) ycsb_exec_coop(YcsbTunedArgs a) {
         stage_init(tab, a.stage_entries);
         __syncthreads();
     }
-    coop_exec_loop<kStage, kFilter, kDedupe, kReads>(a, tab, sbits, srank, kReads && !kStage ? row_scratch<BS>() : nullptr, tag);
+    coop_exec_loop<kStage, kFilter, kDedupe, kReads, BS>(a, tab, sbits, srank, kReads && !kStage ? row_scratch<BS>() : nullptr, tag);
     if (kStage) {
         __syncthreads();
         const uint32_t ops = stage_flush(tab, a.stage_entries, a.reg, tag, a.bucket_counts);
@@ -1011,51 +1070,12 @@ __global__ void __launch_bounds__(BS) ycsb_exec_coop(YcsbTunedArgs a) {
     }
 }
 
-// Shared memory layout: [dig: tile u64][fl: tile u32][stage table]
-__host__ __device__ __forceinline__ size_t ycsb_smem_bytes(uint32_t tile, uint32_t threads, uint32_t stage_entries) {
-    (void)threads;
-    const size_t a = ((size_t)tile * 8 + 15) / 16 * 16;
-    const size_t b = ((size_t)tile * 4 + 15) / 16 * 16;
-    return a + b + (size_t)stage_entries * sizeof(StageEnt);
-}
-
-struct SmemPtrs {
-    unsigned long long *dig;
-    uint32_t *fl;
-    StageEnt *tab;
-};
-__device__ __forceinline__ SmemPtrs carve(char *base, uint32_t tile) {
-    SmemPtrs p;
-    const size_t a = ((size_t)tile * 8 + 15) / 16 * 16;
-    const size_t b = ((size_t)tile * 4 + 15) / 16 * 16;
-    p.dig = reinterpret_cast<unsigned long long *>(base);
-    p.fl = reinterpret_cast<uint32_t *>(base + a);
-    p.tab = reinterpret_cast<StageEnt *>(base + a + b);
-    return p;
-}
-
-template <bool kStage>
-__global__ void __launch_bounds__(512) ycsb_exec_tuned(YcsbTunedArgs a) {
-    extern __shared__ __align__(16) char smem[];
-    const SmemPtrs p = carve(smem, a.tile);
-    const uint64_t tag = slot_tag(a.ctl->epoch);
-    if (kStage) {
-        stage_init(p.tab, a.stage_entries);
-        __syncthreads();
-    }
-    exec_tiles<kStage>(a, p.dig, p.tab, tag);
-    if (kStage) {
-        __syncthreads();
-        const uint32_t ops = stage_flush(p.tab, a.stage_entries, a.reg, tag, a.bucket_counts);
-        if (ops) red_add_u64(&a.st->staged_ops, ops);
-    }
-}
-
+// Registers for three blocks of 512 an SM (two when rows are gathered here).
 template <int kLate>
-__global__ void __launch_bounds__(512) ycsb_checkwb_tuned(YcsbTunedArgs a) {
+__global__ void __launch_bounds__(512, kLate == 1 ? 2 : 3) ycsb_checkwb_tuned(YcsbTunedArgs a) {
     extern __shared__ __align__(16) char smem[];
-    const SmemPtrs p = carve(smem, a.tile);
-    checkwb_tiles<kLate>(a, p.fl, kLate == 1 ? row_scratch<512>() : nullptr, a.ctl->epoch);
+    const SmemPtrs p = carve(smem, a.tile, a.stride);
+    checkwb_tiles<kLate>(a, p, kLate == 1 ? row_scratch<512>() : nullptr, a.ctl->epoch);
     if (!kLate) finish_batch<false>(a.ctl);
 }
 
@@ -1144,14 +1164,14 @@ __global__ void __launch_bounds__(BS) ycsb_writeback_list(YcsbTunedArgs a) {
 // One cooperative kernel per batch: execute+register, grid barrier, check +
 // write-back.  The barrier wait is bounded (grid_barrier); once a wait has
 // run out, a block runs no further phase and calls no further barrier.
-// With late reads (kLate, which needs a.lpt != 0): execute registers only,
+// With late reads (kLate): execute registers only,
 // then check + reads, a second grid barrier, and the write-back.  Phases
 // after the first load what earlier phases wrote with coherent loads
-// (kCoh = true above; checkwb_tiles reads slots with ld.global.cg, at L2).
+// (kCoh = true above), but for the slots in checkwb_tiles.
 template <bool kStage, bool kLate, int BS>
 __device__ __forceinline__ void ycsb_persistent_body(const YcsbTunedArgs &a) {
     extern __shared__ __align__(16) char smem[];
-    const SmemPtrs p = carve(smem, a.tile);
+    const SmemPtrs p = carve(smem, a.tile, a.stride);
     RowScratch *ws = row_scratch<BS>();
     const uint32_t epoch = a.ctl->epoch;
     const uint64_t tag = slot_tag(epoch);
@@ -1173,12 +1193,9 @@ __device__ __forceinline__ void ycsb_persistent_body(const YcsbTunedArgs &a) {
         stage_init(p.tab, a.stage_entries);
         __syncthreads();
     }
-    if (a.lpt) {
-        if (a.filter) coop_exec_loop<kStage, true, true, !kLate>(a, p.tab, a.stage_bits, a.stage_rank, ws, tag);
-        else coop_exec_loop<kStage, false, true, !kLate>(a, p.tab, a.stage_bits, a.stage_rank, ws, tag);
-    } else if (!kLate) {
-        exec_tiles<kStage>(a, p.dig, p.tab, tag);
-    }
+    constexpr int kDedupe = kStage ? DEDUPE_WARP : DEDUPE_BLOCK;
+    if (a.filter) coop_exec_loop<kStage, true, kDedupe, !kLate, BS>(a, p.tab, a.stage_bits, a.stage_rank, ws, tag);
+    else coop_exec_loop<kStage, false, kDedupe, !kLate, BS>(a, p.tab, a.stage_bits, a.stage_rank, ws, tag);
     if (kStage) {
         __syncthreads();
         const uint32_t ops = stage_flush(p.tab, a.stage_entries, a.reg, tag, a.bucket_counts);
@@ -1186,9 +1203,9 @@ __device__ __forceinline__ void ycsb_persistent_body(const YcsbTunedArgs &a) {
     }
     bool ok = grid_barrier(a.ctl);
     if (ok) {
-        if (!kLate) checkwb_tiles<0>(a, p.fl, ws, epoch);
-        else if (a.late == 2u) checkwb_tiles<2>(a, p.fl, ws, epoch);
-        else checkwb_tiles<1>(a, p.fl, ws, epoch);
+        if (!kLate) checkwb_tiles<0>(a, p, ws, epoch);
+        else if (a.late == 2u) checkwb_tiles<2>(a, p, ws, epoch);
+        else checkwb_tiles<1>(a, p, ws, epoch);
     }
     if (kLate) {
         if (a.late == 2u) {
@@ -1278,14 +1295,16 @@ static void launch_fast_t(ltpg_ctx *c, const YcsbTunedArgs &a, bool stage, uint3
 template <bool kReads, int BS>
 static void (*coop_kernel(int sel))(YcsbTunedArgs) {
     switch (sel) {
-    case 0: return ycsb_exec_coop<false, false, false, kReads, BS>;
-    case 1: return ycsb_exec_coop<false, false, true, kReads, BS>;
-    case 2: return ycsb_exec_coop<false, true, false, kReads, BS>;
-    case 3: return ycsb_exec_coop<false, true, true, kReads, BS>;
-    case 4: return ycsb_exec_coop<true, false, false, kReads, BS>;
-    case 5: return ycsb_exec_coop<true, false, true, kReads, BS>;
-    case 6: return ycsb_exec_coop<true, true, false, kReads, BS>;
-    default: return ycsb_exec_coop<true, true, true, kReads, BS>;
+    case 0: return ycsb_exec_coop<false, false, DEDUPE_NONE, kReads, BS>;
+    case 1: return ycsb_exec_coop<false, false, DEDUPE_WARP, kReads, BS>;
+    case 2: return ycsb_exec_coop<false, true, DEDUPE_NONE, kReads, BS>;
+    case 3: return ycsb_exec_coop<false, true, DEDUPE_WARP, kReads, BS>;
+    case 4: return ycsb_exec_coop<true, false, DEDUPE_NONE, kReads, BS>;
+    case 5: return ycsb_exec_coop<true, false, DEDUPE_WARP, kReads, BS>;
+    case 6: return ycsb_exec_coop<true, true, DEDUPE_NONE, kReads, BS>;
+    case 7: return ycsb_exec_coop<true, true, DEDUPE_WARP, kReads, BS>;
+    case 8: return ycsb_exec_coop<false, false, DEDUPE_BLOCK, kReads, BS>;
+    default: return ycsb_exec_coop<false, true, DEDUPE_BLOCK, kReads, BS>;
     }
 }
 
@@ -1293,7 +1312,12 @@ static void (*coop_kernel(int sel))(YcsbTunedArgs) {
 static void launch_coop(ltpg_ctx *c, const YcsbTunedArgs &a, bool stage, bool reads) {
     const LaunchCfg &L = c->launch_y;
     const size_t smem = stage ? 2 * STAGE_WORDS * sizeof(uint32_t) + (size_t)a.stage_entries * sizeof(StageEnt) : 0;
-    const int sel = (stage ? 4 : 0) | (L.filter ? 2 : 0) | (L.dedupe ? 1 : 0);
+    const uint64_t nw = (uint64_t)a.B * a.lpt;
+    // Up to about eight waves a block registers a key once whatever is asked for
+    // (65,536 x 10: theta 0.99 29 -> 21 us, 0 and 0.6 within 1 us); beyond, the barrier
+    // per step costs more than it saves (2^18 x 10 at theta 0.6: 48 -> 53 us).
+    const bool few_waves = nw <= 8192ull * c->sm_count;
+    const int sel = !stage && few_waves ? (L.filter ? 9 : 8) : (stage ? 4 : 0) | (L.filter ? 2 : 0) | (L.dedupe ? 1 : 0);
     void (*k)(YcsbTunedArgs) = with_block(L.block, [&](auto bs) {
         constexpr int BS = decltype(bs)::value;
         return reads ? coop_kernel<true, BS>(sel) : coop_kernel<false, BS>(sel);
@@ -1305,7 +1329,6 @@ static void launch_coop(ltpg_ctx *c, const YcsbTunedArgs &a, bool stage, bool re
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, (int)threads, smem);
     if (per_sm < 1) per_sm = 1;
     if (L.blocks_per_sm && (int)L.blocks_per_sm < per_sm) per_sm = (int)L.blocks_per_sm;
-    const uint64_t nw = (uint64_t)a.B * a.lpt;
     const uint32_t grid = (uint32_t)std::min<uint64_t>((nw + threads - 1) / threads, (uint64_t)per_sm * c->sm_count);
     k<<<grid, threads, smem, c->stream>>>(a);
 }
@@ -1358,28 +1381,22 @@ static cudaError_t launch_write_first(ltpg_ctx *c, const YcsbTunedArgs &a) {
     return with_block(c->launch_y.block, [&](auto bs) { return launch_write_first_t<decltype(bs)::value>(c, a); });
 }
 
-// Launch shapes of the execute phase, by ops_per_thread: 1 = cooperative row
-// reads (ycsb_exec_coop, any stride <= 32), 2 / 4 = per-thread row reads
-// (ycsb_exec_fast, stride / ops a power of two); 8 = block tiles
-// (ycsb_exec_tuned), which serve every stride.
-static bool launch_fast_exec(ltpg_ctx *c, const YcsbTunedArgs &a, bool stage) {
-    const uint32_t opt = c->launch_y.per_thread ? c->launch_y.per_thread : 4u;
-    if (opt >= 8) return false;
-    if (opt == 1 && a.lpt) {
-        launch_coop(c, a, stage, true);
-        return true;
-    }
-    const uint32_t ops = std::max<uint32_t>(2u, std::min<uint32_t>(opt, 4u));
-    if (a.stride % ops) return false;
+// Launch shapes of the execute phase, by ops_per_thread: 2 / 4 = per-thread row
+// reads (ycsb_exec_fast) where stride / ops is a power of two, otherwise
+// cooperative row reads (ycsb_exec_coop).
+static void launch_exec(ltpg_ctx *c, const YcsbTunedArgs &a, bool stage) {
+    const uint32_t ops = c->launch_y.per_thread ? c->launch_y.per_thread : 4u;
     const uint32_t lpt = a.stride / ops;
-    if (lpt == 0 || lpt > 32 || (lpt & (lpt - 1))) return false;
+    if ((ops != 2u && ops != 4u) || (lpt & (lpt - 1))) {
+        launch_coop(c, a, stage, true);
+        return;
+    }
     with_block(c->launch_y.block, [&](auto bs) {
         constexpr int BS = decltype(bs)::value;
         if (ops == 2) launch_fast_t<2, BS>(c, a, stage, lpt);
         else launch_fast_t<4, BS>(c, a, stage, lpt);
         return 0;
     });
-    return true;
 }
 
 cudaError_t ycsb_run_tuned(ltpg_ctx *c, Slot &s, int mode) {
@@ -1394,12 +1411,9 @@ cudaError_t ycsb_run_tuned(ltpg_ctx *c, Slot &s, int mode) {
     a.B = s.n_txn;
     a.k = s.k;
     a.stride = s.stride;
-    a.lpt = 0;
-    if (s.stride <= 32) {
-        a.lpt = 1;
-        while (a.lpt < s.stride) a.lpt <<= 1;
-    }
-    a.tile = tuned_tile(s.stride, threads, per_thread);
+    a.lpt = 4;
+    while (a.lpt < s.stride) a.lpt <<= 1;
+    a.tile = tuned_tile(s.stride, threads, per_thread);  // at most; small batches take less, below
     a.rows = c->ycsb.rows;
     a.n = c->ycsb.n;
     a.reg = c->ycsb.reg;
@@ -1416,10 +1430,9 @@ cudaError_t ycsb_run_tuned(ltpg_ctx *c, Slot &s, int mode) {
     a.ways = L.ways ? L.ways : 4u;
     // with the predictor counting but staging off, the staging table is empty
     a.stage_entries = (stage && c->stage_on) ? STAGE_MAX_ENTRIES / a.ways * a.ways : 0u;
-    // late reads need the one-op-per-lane layout (stride <= 32); write-first
-    // registration has no staging path (with staging it reads late in a
-    // kernel of their own)
-    uint32_t late_mode = a.lpt ? L.late_reads : 0u;
+    // write-first registration has no staging path (with staging it reads late
+    // in a kernel of their own)
+    uint32_t late_mode = L.late_reads;
     if (late_mode == 3u && stage) late_mode = 2u;
     const bool late = late_mode != 0u;
     a.filter = L.filter;
@@ -1428,32 +1441,38 @@ cudaError_t ycsb_run_tuned(ltpg_ctx *c, Slot &s, int mode) {
     a.upd = c->ycsb.upd;
     a.upd_cap = c->ycsb.upd_cap;
     a.vals_cap = s.cap_vals;
-    const size_t smem = ycsb_smem_bytes(a.tile, threads, a.stage_entries);
-    const size_t smem_cwb = ycsb_smem_bytes(a.tile, threads, 0);  // check + write-back needs no staging table
+    const size_t smem = ycsb_smem_bytes(a.tile, a.stride, a.stage_entries);
+    const size_t smem_cwb = ycsb_smem_bytes(a.tile, a.stride, 0);  // check + write-back needs no staging table
     cudaError_t e = cudaMemsetAsync(s.stats, 0, sizeof(DevStats), c->stream);
     if (e != cudaSuccess) return e;
     // write-first: the writer bitmap starts empty for every batch
     if (late_mode == 3u &&
         (e = cudaMemsetAsync(a.wbits, 0, (a.n + 31) / 32 * sizeof(uint32_t), c->stream)) != cudaSuccess)
         return e;
-    auto exec_k = stage ? ycsb_exec_tuned<true> : ycsb_exec_tuned<false>;
     auto pers_k = stage ? (late ? ycsb_persistent<true, true> : ycsb_persistent<true, false>)
                         : (late ? (threads <= 256 ? ycsb_persistent_late_x6 : ycsb_persistent<false, true>)
                                 : ycsb_persistent<false, false>);
     auto cwb_k = !late ? ycsb_checkwb_tuned<0> : late_mode == 1u ? ycsb_checkwb_tuned<1> : ycsb_checkwb_tuned<2>;
     // above 48 KB of static + dynamic shared memory a kernel must opt in
-    for (const void *k : {(const void *)exec_k, (const void *)cwb_k, (const void *)pers_k})
+    for (const void *k : {(const void *)cwb_k, (const void *)pers_k})
         if (smem + static_smem(k) > 48 * 1024)
             cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const bool persistent = mode == LTPG_MODE_PERSISTENT;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mode == LTPG_MODE_PERSISTENT ? pers_k : exec_k,
-                                                      (int)threads, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent ? pers_k : cwb_k, (int)threads,
+                                                      persistent ? smem : smem_cwb);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    if (L.blocks_per_sm && (int)L.blocks_per_sm < per_sm) per_sm = (int)L.blocks_per_sm;
+    if (persistent && L.blocks_per_sm && (int)L.blocks_per_sm < per_sm) per_sm = (int)L.blocks_per_sm;
+    // A batch of less than one wave is spread over all resident blocks: the
+    // kernels are chains of dependent accesses, which more threads shorten.
+    const uint32_t resident = (uint32_t)(per_sm * c->sm_count);
+    a.tile = std::min(a.tile, ((a.B + resident - 1) / resident + 31u) / 32u * 32u);
     const uint32_t n_tiles = (a.B + a.tile - 1) / a.tile;
-    const uint32_t grid = std::min<uint32_t>(n_tiles, (uint32_t)(per_sm * c->sm_count));
-    if (mode == LTPG_MODE_PERSISTENT) {
+    if (persistent) {
+        // a lane per op in the first phase
+        const uint64_t blocks = std::max<uint64_t>(n_tiles, ((uint64_t)a.B * a.lpt + threads - 1) / threads);
+        const uint32_t grid = (uint32_t)std::min<uint64_t>(resident, blocks);
         prof_mark(c, 0);
         void *args[] = {&a};
         count_launch(c);
@@ -1466,15 +1485,11 @@ cudaError_t ycsb_run_tuned(ltpg_ctx *c, Slot &s, int mode) {
     prof_mark(c, 0);
     count_launch(c);
     if (late) launch_coop(c, a, stage, false);
-    else if (!launch_fast_exec(c, a, stage)) exec_k<<<grid, threads, smem, c->stream>>>(a);
+    else launch_exec(c, a, stage);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     prof_mark(c, 1);
     count_launch(c);
-    int per_sm_cwb = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_cwb, cwb_k, (int)threads, smem_cwb);
-    if (e != cudaSuccess) return e;
-    if (per_sm_cwb < 1) per_sm_cwb = 1;
-    const uint32_t grid_cwb = std::min<uint32_t>(n_tiles, (uint32_t)(per_sm_cwb * c->sm_count));
+    const uint32_t grid_cwb = std::min(n_tiles, resident);
     cwb_k<<<grid_cwb, threads, smem_cwb, c->stream>>>(a);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     prof_mark(c, 2);
