@@ -504,6 +504,7 @@ __device__ __forceinline__ void wf_register_reads(const YcsbTunedArgs &a, uint32
 
 template <int BS>
 __global__ void __launch_bounds__(BS) ycsb_wf_writes(YcsbTunedArgs a) {
+    clear_stats(a.st);
     wf_register_writes<false>(a, slot_tag(a.ctl->epoch));
 }
 
@@ -756,6 +757,8 @@ __global__ void __launch_bounds__(BS) ycsb_exec_fast(YcsbTunedArgs a, uint32_t l
     StageEnt *tab = reinterpret_cast<StageEnt *>(smem);
     const uint64_t tag = slot_tag(a.ctl->epoch);
     const uint32_t lane = threadIdx.x & 31;
+    let_next_start();
+    if (!kStage) clear_stats(a.st);
     if (kStage) {
         stage_init(tab, a.stage_entries);
         __syncthreads();
@@ -1054,6 +1057,8 @@ __global__ void __launch_bounds__(BS) ycsb_exec_coop(YcsbTunedArgs a) {
     uint32_t *srank = sbits + STAGE_WORDS;
     StageEnt *tab = reinterpret_cast<StageEnt *>(srank + STAGE_WORDS);
     const uint64_t tag = slot_tag(a.ctl->epoch);
+    let_next_start();
+    if (!kStage) clear_stats(a.st);
     if (kStage) {
         for (uint32_t i = threadIdx.x; i < STAGE_WORDS; i += blockDim.x) {
             sbits[i] = __ldg(a.stage_bits + i);
@@ -1075,6 +1080,7 @@ template <int kLate>
 __global__ void __launch_bounds__(512, kLate == 1 ? 2 : 3) ycsb_checkwb_tuned(YcsbTunedArgs a) {
     extern __shared__ __align__(16) char smem[];
     const SmemPtrs p = carve(smem, a.tile, a.stride);
+    wait_for_previous();
     checkwb_tiles<kLate>(a, p, kLate == 1 ? row_scratch<512>() : nullptr, a.ctl->epoch);
     if (!kLate) finish_batch<false>(a.ctl);
 }
@@ -1175,6 +1181,7 @@ __device__ __forceinline__ void ycsb_persistent_body(const YcsbTunedArgs &a) {
     RowScratch *ws = row_scratch<BS>();
     const uint32_t epoch = a.ctl->epoch;
     const uint64_t tag = slot_tag(epoch);
+    if (!kStage) clear_stats(a.st);
     if (kLate && !kStage && a.late == 3u) {  // write-first: five phases, four grid barriers
         wf_register_writes<true>(a, tag);
         bool ok = grid_barrier(a.ctl);
@@ -1308,16 +1315,22 @@ static void (*coop_kernel(int sel))(YcsbTunedArgs) {
     }
 }
 
+// A batch of up to about eight waves of lanes.  In one, a block registers a key
+// once whatever is asked for (65,536 x 10: theta 0.99 29 -> 21 us, 0 and 0.6
+// within 1 us); beyond, the barrier per step costs more than it saves (2^18 x 10
+// at theta 0.6: 48 -> 53 us).  And the check's launch overlaps the execute
+// kernel (65,536 x 10: 29.5 -> 27 us a batch); beyond, its early blocks are in
+// the way (2^20 x 10: 240 -> 242 us; with staging 414 -> 427).
+static bool few_waves(const ltpg_ctx *c, const YcsbTunedArgs &a) {
+    return (uint64_t)a.B * a.lpt <= 8192ull * c->sm_count;
+}
+
 // reads = false: registration only (late reads)
 static void launch_coop(ltpg_ctx *c, const YcsbTunedArgs &a, bool stage, bool reads) {
     const LaunchCfg &L = c->launch_y;
     const size_t smem = stage ? 2 * STAGE_WORDS * sizeof(uint32_t) + (size_t)a.stage_entries * sizeof(StageEnt) : 0;
     const uint64_t nw = (uint64_t)a.B * a.lpt;
-    // Up to about eight waves a block registers a key once whatever is asked for
-    // (65,536 x 10: theta 0.99 29 -> 21 us, 0 and 0.6 within 1 us); beyond, the barrier
-    // per step costs more than it saves (2^18 x 10 at theta 0.6: 48 -> 53 us).
-    const bool few_waves = nw <= 8192ull * c->sm_count;
-    const int sel = !stage && few_waves ? (L.filter ? 9 : 8) : (stage ? 4 : 0) | (L.filter ? 2 : 0) | (L.dedupe ? 1 : 0);
+    const int sel = !stage && few_waves(c, a) ? (L.filter ? 9 : 8) : (stage ? 4 : 0) | (L.filter ? 2 : 0) | (L.dedupe ? 1 : 0);
     void (*k)(YcsbTunedArgs) = with_block(L.block, [&](auto bs) {
         constexpr int BS = decltype(bs)::value;
         return reads ? coop_kernel<true, BS>(sel) : coop_kernel<false, BS>(sel);
@@ -1443,7 +1456,8 @@ cudaError_t ycsb_run_tuned(ltpg_ctx *c, Slot &s, int mode) {
     a.vals_cap = s.cap_vals;
     const size_t smem = ycsb_smem_bytes(a.tile, a.stride, a.stage_entries);
     const size_t smem_cwb = ycsb_smem_bytes(a.tile, a.stride, 0);  // check + write-back needs no staging table
-    cudaError_t e = cudaMemsetAsync(s.stats, 0, sizeof(DevStats), c->stream);
+    // a staging execute kernel adds to the counters; otherwise the first kernel clears them
+    cudaError_t e = stage ? cudaMemsetAsync(s.stats, 0, sizeof(DevStats), c->stream) : cudaSuccess;
     if (e != cudaSuccess) return e;
     // write-first: the writer bitmap starts empty for every batch
     if (late_mode == 3u &&
@@ -1490,8 +1504,8 @@ cudaError_t ycsb_run_tuned(ltpg_ctx *c, Slot &s, int mode) {
     prof_mark(c, 1);
     count_launch(c);
     const uint32_t grid_cwb = std::min(n_tiles, resident);
-    cwb_k<<<grid_cwb, threads, smem_cwb, c->stream>>>(a);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = launch_next(cwb_k, !stage && few_waves(c, a), grid_cwb, threads, smem_cwb, c->stream, a);
+    if (e != cudaSuccess) return e;
     prof_mark(c, 2);
     if (late_mode == 2u) {
         count_launch(c);
