@@ -50,6 +50,7 @@ void free_slot(Slot &s) {
     dev_free(s.stats);
     if (s.copied) cudaEventDestroy(s.copied);
     if (s.done) cudaEventDestroy(s.done);
+    if (s.left) cudaFreeHost(s.left);
     s = Slot{};
 }
 
@@ -78,10 +79,12 @@ int ensure_outputs(ltpg_ctx *c, Slot &s, uint64_t n) {
     return LTPG_OK;
 }
 
-// Reads and clears the device error word; call after a synchronisation.
+// Waits for the stream, then reads and clears the device error word.  The copy
+// is queued behind the stream's work, so that one wait does for both.
 int check_device_error(ltpg_ctx *c) {
     DevCtl h;
-    CK(cudaMemcpy(&h, c->ctl, sizeof h, cudaMemcpyDeviceToHost), "read control block");
+    CK(cudaMemcpyAsync(&h, c->ctl, sizeof h, cudaMemcpyDeviceToHost, c->stream), "read control block");
+    CK(cudaStreamSynchronize(c->stream), "stream synchronize");
     if (h.error == 0) return LTPG_OK;
     const uint32_t error = h.error, index = h.err_index;
     // clear the error and any barrier / completion state a failed kernel left
@@ -233,7 +236,6 @@ void *ltpg_get_stream(ltpg_ctx *c) { return c ? (void *)c->stream : nullptr; }
 
 int ltpg_sync(ltpg_ctx *c) {
     if (!c) return LTPG_ERR_INVALID;
-    CK(cudaStreamSynchronize(c->stream), "stream synchronize");
     return check_device_error(c);
 }
 
@@ -694,7 +696,11 @@ int submit_host(ltpg_ctx *c, uint32_t slot, int mode, uint32_t *host_bitmap, Up 
         CK(cudaMemcpyAsync(host_bitmap, s->bitmap, ((uint64_t)s->n_txn + 31) / 32 * 4, cudaMemcpyDeviceToHost,
                            c->stream),
            "bitmap download");
+    // the control block as the batch leaves it, for the slot's wait
+    if (!s->left) CK(cudaMallocHost((void **)&s->left, sizeof(DevCtl)), "alloc control block copy");
+    CK(cudaMemcpyAsync(s->left, c->ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, c->stream), "read control block");
     CK(cudaEventRecord(s->done, c->stream), "record done");
+    s->submitted = true;
     return LTPG_OK;
 }
 }  // namespace
@@ -732,7 +738,9 @@ int ltpg_host_wait(ltpg_ctx *c, uint32_t slot) {
     Slot *s = get_slot(c, slot);
     if (!s) return c ? fail(c, LTPG_ERR_INVALID, "bad slot") : LTPG_ERR_INVALID;
     if (s->done) CK(cudaEventSynchronize(s->done), "wait for the slot");
-    return check_device_error(c);
+    const bool clean = s->submitted && s->left->error == 0u;
+    s->submitted = false;
+    return clean ? LTPG_OK : check_device_error(c);
 }
 
 // ---- results -----------------------------------------------------------------

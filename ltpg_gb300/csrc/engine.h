@@ -127,6 +127,8 @@ struct Slot {
     // pipelined host calls: the batch's copy is done / the slot's last use
     // (kernels and bitmap download) is done
     cudaEvent_t copied = nullptr, done = nullptr;
+    DevCtl *left = nullptr;  // pinned: the control block as the submitted batch left it
+    bool submitted = false;  // and no wait has looked at it
 };
 
 struct LaunchCfg {

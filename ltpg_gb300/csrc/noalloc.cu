@@ -125,9 +125,9 @@ extern "C" int ltpg_ycsb_batch_noalloc(int device, uint64_t *rows, uint64_t n_re
     ycsb_writeback_plain<<<(n_txn + 255) / 256, 256, 0, s>>>(flags, n_txn, ops, k, stride, val_off, vals, ~0ull,
                                                              rows, n_records, bitmap, d->stats, d->ctl);
     if (cudaGetLastError() != cudaSuccess) return LTPG_ERR_CUDA;
+    uint32_t err = 0;  // copied behind the kernels: one wait for both
+    if (cudaMemcpyAsync(&err, &d->ctl->error, sizeof err, cudaMemcpyDeviceToHost, s) != cudaSuccess) return LTPG_ERR_CUDA;
     if (cudaStreamSynchronize(s) != cudaSuccess) return LTPG_ERR_CUDA;
-    uint32_t err = 0;
-    if (cudaMemcpy(&err, &d->ctl->error, sizeof err, cudaMemcpyDeviceToHost) != cudaSuccess) return LTPG_ERR_CUDA;
     if (err) {
         DevCtl h{};
         if (cudaMemcpy(&h, d->ctl, sizeof h, cudaMemcpyDeviceToHost) != cudaSuccess) return LTPG_ERR_CUDA;

@@ -70,6 +70,7 @@ struct DevSlot {
     bool busy = false;
     cudaEvent_t start = nullptr, done_c = nullptr, done_y = nullptr;
     Pinned c_flags, c_res, y_flags, y_res;  // results, copied back behind the kernels
+    Pinned ctl;                             // and both engines' control blocks as the batch leaves them
     uint64_t first_id = 0;
     uint32_t n = 0, n_c = 0, n_y = 0;
     std::vector<uint32_t> map;      // per request: (index in its part << 1) | (1 for YCSB)
@@ -121,6 +122,7 @@ struct ltpg_server {
     uint64_t committed = 0, batches = 0, waited_for_slot = 0;
     double wait_sum = 0, launch_sum = 0, dev_sum = 0;
     int error = LTPG_OK;
+    bool look = true;  // flush asks the engines for errors: at first, and when a batch left one
 
     double now() const { return std::chrono::duration<double>(Clock::now() - t0).count(); }
 };
@@ -166,6 +168,8 @@ bool complete_oldest(ltpg_server *s, bool block) {
     cudaEventElapsedTime(&ms_c, d.start, d.done_c);
     cudaEventElapsedTime(&ms_y, d.start, d.done_y);
     s->dev_sum += std::max(ms_c, ms_y) * 1e-3;
+    const DevCtl *ctl = d.ctl.as<DevCtl>();
+    s->look |= (d.n_c && ctl[0].error) || (d.n_y && ctl[1].error);
     const uint8_t *cf = d.c_flags.as<uint8_t>(), *yf = d.y_flags.as<uint8_t>();
     const int64_t *cr = d.c_res.as<int64_t>(), *yr = d.y_res.as<int64_t>();
     for (uint32_t i = 0; i < d.n; ++i) {
@@ -235,6 +239,7 @@ int close_batch(ltpg_server *s, bool block) {
         const Slot &es = s->tc->slots[slot];
         cudaMemcpyAsync(d.c_flags.p, es.flags, s->form_c, cudaMemcpyDeviceToHost, s->cs_c);
         cudaMemcpyAsync(d.c_res.p, es.results, (size_t)s->form_c * 8, cudaMemcpyDeviceToHost, s->cs_c);
+        cudaMemcpyAsync(d.ctl.p, s->tc->ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, s->cs_c);
     } else {
         cudaEventRecord(g.up_c, s->cp_c);
         cudaStreamWaitEvent(s->cs_c, d.start, 0);
@@ -253,6 +258,7 @@ int close_batch(ltpg_server *s, bool block) {
         const Slot &es = s->yc->slots[slot];
         cudaMemcpyAsync(d.y_flags.p, es.flags, s->form_y, cudaMemcpyDeviceToHost, s->cs_y);
         cudaMemcpyAsync(d.y_res.p, es.results, (size_t)s->form_y * 8, cudaMemcpyDeviceToHost, s->cs_y);
+        cudaMemcpyAsync(d.ctl.as<DevCtl>() + 1, s->yc->ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, s->cs_y);
     } else {
         cudaEventRecord(g.up_y, s->cp_y);
         cudaStreamWaitEvent(s->cs_y, d.start, 0);
@@ -346,14 +352,17 @@ int submit(ltpg_server *s, const ltpg_request *reqs, uint32_t n, uint64_t *first
     int r = progress(s);
     if (r) return r;
     if (first_id) *first_id = s->next_id;
+    double called = s->now();  // and again after every wait below
     for (uint32_t i = 0; i < n; ++i) {
         const ltpg_request &q = reqs[i];
         if ((r = check_request(s, q))) return r;
-        const double t = t_submit ? t_submit[i] : s->now();
+        const double t = t_submit ? t_submit[i] : called;
         const bool lines_full =
             q.workload == LTPG_WORKLOAD_TPCC && s->form_lines + q.n > s->max_lines;
-        if (s->form_n && (s->form_n >= s->max_batch || lines_full))
+        if (s->form_n && (s->form_n >= s->max_batch || lines_full)) {
             if ((r = close_batch(s, true))) return r;
+            called = s->now();
+        }
         if (s->form_n == 0 && (r = begin_forming(s, t))) return r;
         pack(s, q, t);
     }
@@ -368,6 +377,8 @@ int flush(ltpg_server *s) {
     while (s->in_flight)
         if (!complete_oldest(s, true)) return fail(s, s->error ? s->error : LTPG_ERR_CUDA);
     // device-side errors of the batches (out-of-range keys) are reported here
+    if (!s->look) return LTPG_OK;
+    s->look = false;
     int r1 = ltpg_sync(s->tc), r2 = ltpg_sync(s->yc);
     if (r1 || r2) return fail(s, r1 ? r1 : r2);
     return LTPG_OK;
@@ -460,7 +471,8 @@ int ltpg_server_open(ltpg_ctx *tc, ltpg_ctx *yc, const ltpg_server_cfg *cfg, ltp
              cudaEventCreateWithFlags(&g.up_y, cudaEventDisableTiming) == cudaSuccess;
     }
     for (auto &d : s->dev) {
-        ok = ok && d.c_flags.reserve(m) && d.c_res.reserve(m * 8) && d.y_flags.reserve(m) && d.y_res.reserve(m * 8);
+        ok = ok && d.c_flags.reserve(m) && d.c_res.reserve(m * 8) && d.y_flags.reserve(m) && d.y_res.reserve(m * 8) &&
+             d.ctl.reserve(2 * sizeof(DevCtl));
         ok = ok && cudaEventCreate(&d.start) == cudaSuccess && cudaEventCreate(&d.done_c) == cudaSuccess &&
              cudaEventCreate(&d.done_y) == cudaSuccess;
     }
