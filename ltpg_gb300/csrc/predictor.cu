@@ -16,6 +16,7 @@
 // The forward pass runs on the tensor cores (mma.sync m16n8k16, BF16 inputs,
 // FP32 accumulators); backward and Adam are FP32.  The predictor only picks
 // the staged set, which changes speed, never a commit decision.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
 #include <cstring>
@@ -24,6 +25,8 @@
 #include "stage.cuh"
 
 namespace ltpg {
+
+namespace cg = cooperative_groups;
 
 constexpr int PH = 64;            // hidden width
 constexpr int PF = 4;             // features (batches of history)
@@ -55,14 +58,11 @@ __device__ __forceinline__ void mma_bf16(float *d, const uint32_t *a, const uint
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// Features of bucket b: log1p of its counts in the 4 ring slots ending at
-// `newest` (oldest first).
-__device__ __forceinline__ void features(const uint32_t *ring, uint32_t newest, uint32_t b, float *x) {
-#pragma unroll
-    for (int f = 0; f < PF; ++f) {
-        const uint32_t slot = (newest + P_RING - (PF - 1 - f)) % P_RING;
-        x[f] = log1pf((float)ring[slot * STAGE_BUCKETS + b]);
-    }
+// Feature f of bucket b: log1p of its count in the f-th of the 4 ring slots
+// ending at `newest` (oldest first).
+__device__ __forceinline__ float feature(const uint32_t *ring, uint32_t newest, uint32_t b, uint32_t f) {
+    const uint32_t slot = (newest + P_RING - (PF - 1 - f)) % P_RING;
+    return log1pf((float)ring[slot * STAGE_BUCKETS + b]);
 }
 
 // ---- forward on tensor cores ----------------------------------------------------
@@ -76,14 +76,22 @@ __device__ __forceinline__ void features(const uint32_t *ring, uint32_t newest, 
 //         also stores X, H1, H2, Y, T for the backward pass.
 // mode 2: x given in `xin` [n][4] (tests), writes y.  mode 3: x given in `xin`,
 //         stores X, H1, H2, Y like mode 1 (the gradient test sets T).
+// A warp has little to do, so what surrounds it bounds it: the weights come in
+// 16-byte loads, their rows are padded so that the eight rows of a fragment lie
+// in different banks (unpadded they met in one), and the four lanes of a row
+// take one feature each (each took all four).  One tile a warp.  65,536 buckets
+// 20 -> 11 us, 4,096 samples 14 -> 9.4 us (cold).
+constexpr int W1_ROW = 24, W2_ROW = 72;  // padded rows in shared memory, BF16
 __global__ void __launch_bounds__(256) pred_forward(PredDev p, uint32_t n, int mode, const float *__restrict__ xin,
                                                     float *__restrict__ yout) {
-    __shared__ __align__(16) __nv_bfloat16 w1s[PH * 16];
-    __shared__ __align__(16) __nv_bfloat16 w2s[PH * PH];
+    __shared__ __align__(16) __nv_bfloat16 w1s[PH * W1_ROW];
+    __shared__ __align__(16) __nv_bfloat16 w2s[PH * W2_ROW];
     __shared__ float b1s[PH], b2s[PH], w3s[PH];
     __shared__ float b3s;
-    for (int i = threadIdx.x; i < PH * 16; i += blockDim.x) w1s[i] = p.w1b[i];
-    for (int i = threadIdx.x; i < PH * PH; i += blockDim.x) w2s[i] = p.w2b[i];
+    for (int i = threadIdx.x; i < PH * 2; i += blockDim.x)
+        *reinterpret_cast<uint4 *>(w1s + i / 2 * W1_ROW + i % 2 * 8) = reinterpret_cast<const uint4 *>(p.w1b)[i];
+    for (int i = threadIdx.x; i < PH * PH / 8; i += blockDim.x)
+        *reinterpret_cast<uint4 *>(w2s + i / 8 * W2_ROW + i % 8 * 8) = reinterpret_cast<const uint4 *>(p.w2b)[i];
     for (int i = threadIdx.x; i < PH; i += blockDim.x) {
         b1s[i] = p.param[P_B1 + i];
         b2s[i] = p.param[P_B2 + i];
@@ -99,35 +107,37 @@ __global__ void __launch_bounds__(256) pred_forward(PredDev p, uint32_t n, int m
     for (uint32_t s0 = warp * 16; s0 < n; s0 += n_warps * 16) {
         // sample ids of rows g and g + 8
         uint32_t sid[2] = {s0 + g, s0 + g + 8};
-        float xr[2][PF], tr[2] = {0.f, 0.f};
+        float xq[2], tr[2] = {0.f, 0.f};  // this lane's feature (q) of both rows
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const uint32_t s = sid[h];
-#pragma unroll
-            for (int f = 0; f < PF; ++f) xr[h][f] = 0.f;
+            xq[h] = 0.f;
             if (s >= n) continue;
             if (mode == 2 || mode == 3) {
-#pragma unroll
-                for (int f = 0; f < PF; ++f) xr[h][f] = xin[s * PF + f];
+                xq[h] = xin[s * PF + q];
             } else if (mode == 1) {
                 const uint32_t b = (s * 16u + (step & 15u)) & (STAGE_BUCKETS - 1u);  // rotating 1/16 of buckets
-                features(p.ring, (newest + P_RING - 1) % P_RING, b, xr[h]);
-                tr[h] = log1pf((float)p.ring[newest * STAGE_BUCKETS + b]);
+                xq[h] = feature(p.ring, (newest + P_RING - 1) % P_RING, b, q);
+                if (q == 0) tr[h] = log1pf((float)p.ring[newest * STAGE_BUCKETS + b]);
             } else {
-                features(p.ring, newest, s, xr[h]);
+                xq[h] = feature(p.ring, newest, s, q);
             }
         }
         // A fragment of layer 1: features are k = 0..3 (lanes q = 0, 1)
         uint32_t a1[4];
-        a1[0] = q == 0 ? pack_bf16(xr[0][0], xr[0][1]) : q == 1 ? pack_bf16(xr[0][2], xr[0][3]) : 0u;
-        a1[1] = q == 0 ? pack_bf16(xr[1][0], xr[1][1]) : q == 1 ? pack_bf16(xr[1][2], xr[1][3]) : 0u;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const float lo = __shfl_sync(FULL, xq[h], (lane & 28u) | ((2u * q) & 3u));
+            const float hi = __shfl_sync(FULL, xq[h], (lane & 28u) | ((2u * q + 1u) & 3u));
+            a1[h] = q < 2u ? pack_bf16(lo, hi) : 0u;
+        }
         a1[2] = 0u;
         a1[3] = 0u;
         float h1[8][4];
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
             h1[nt][0] = h1[nt][1] = h1[nt][2] = h1[nt][3] = 0.f;
-            const __nv_bfloat16 *wr = w1s + (nt * 8 + g) * 16;
+            const __nv_bfloat16 *wr = w1s + (nt * 8 + g) * W1_ROW;
             uint32_t b[2] = {*reinterpret_cast<const uint32_t *>(wr + q * 2),
                              *reinterpret_cast<const uint32_t *>(wr + 8 + q * 2)};
             mma_bf16(h1[nt], a1, b);
@@ -147,7 +157,7 @@ __global__ void __launch_bounds__(256) pred_forward(PredDev p, uint32_t n, int m
                              pack_bf16(h1[2 * kb + 1][2], h1[2 * kb + 1][3])};
 #pragma unroll
             for (int nt = 0; nt < 8; ++nt) {
-                const __nv_bfloat16 *wr = w2s + (nt * 8 + g) * PH + kb * 16;
+                const __nv_bfloat16 *wr = w2s + (nt * 8 + g) * W2_ROW + kb * 16;
                 uint32_t b[2] = {*reinterpret_cast<const uint32_t *>(wr + q * 2),
                                  *reinterpret_cast<const uint32_t *>(wr + 8 + q * 2)};
                 mma_bf16(h2[nt], a, b);
@@ -177,9 +187,8 @@ __global__ void __launch_bounds__(256) pred_forward(PredDev p, uint32_t n, int m
             for (int h = 0; h < 2; ++h) {
                 const uint32_t s = sid[h];
                 if (s >= n) continue;
+                X[s * PF + q] = xq[h];
                 if (q == 0) {
-#pragma unroll
-                    for (int f = 0; f < PF; ++f) X[s * PF + f] = xr[h][f];
                     Y[s] = h ? y1 : y0;
                     if (mode == 1) T[s] = tr[h];
                 }
@@ -187,10 +196,10 @@ __global__ void __launch_bounds__(256) pred_forward(PredDev p, uint32_t n, int m
                 for (int nt = 0; nt < 8; ++nt) {
                     const int c = nt * 8 + q * 2;
                     // layer 2 consumed BF16(h1): keep that value for the gradient
-                    H1[s * PH + c] = __bfloat162float(__float2bfloat16_rn(h1[nt][2 * h]));
-                    H1[s * PH + c + 1] = __bfloat162float(__float2bfloat16_rn(h1[nt][2 * h + 1]));
-                    H2[s * PH + c] = h2[nt][2 * h];
-                    H2[s * PH + c + 1] = h2[nt][2 * h + 1];
+                    *reinterpret_cast<float2 *>(H1 + s * PH + c) =
+                        make_float2(__bfloat162float(__float2bfloat16_rn(h1[nt][2 * h])),
+                                    __bfloat162float(__float2bfloat16_rn(h1[nt][2 * h + 1])));
+                    *reinterpret_cast<float2 *>(H2 + s * PH + c) = make_float2(h2[nt][2 * h], h2[nt][2 * h + 1]);
                 }
             }
         } else if (q == 0) {
@@ -206,92 +215,123 @@ __global__ void __launch_bounds__(256) pred_forward(PredDev p, uint32_t n, int m
 // dz2[s][j] = 2 (y - t) / S * w3[j] * [h2 > 0];  dh1[s][k] = sum_j dz2[s][j] W2[j][k];
 // dz1 = dh1 * [h1 > 0].  The weights used are the BF16 copies the forward used.
 // One kernel: a block walks tiles of PB samples; per tile dz2 and dz1 are made
-// in shared memory, and each thread adds the tile's terms of its parameters
-// (tid, tid + 256, ...) to registers; the block adds its sums to the global
-// gradient once at the end, and its share of the squared error to loss[1].
-constexpr int PB = 16;                                  // samples per tile
-constexpr int P_PER_THREAD = (P_NPARAM + 255) / 256;    // parameters per thread (256 threads)
+// in shared memory, and each thread adds the tile's terms of its parameters to
+// registers: a 4 x 4 block of W2, one of W1 and at most one of the others.  The
+// block adds its sums to the global gradient once at the end, and its share of
+// the squared error to loss[1].  Shared-memory reads bound it: the 4 x 4 block
+// reads two 16-byte vectors for 16 products, where one parameter at a time read
+// two words for each (4,096 samples 36 -> 11 us).
+constexpr int PB = 16;       // samples per tile
+constexpr int PR = PH + 4;   // padded row of a tile
 
 __global__ void __launch_bounds__(256) pred_backward(PredDev p, uint32_t S) {
     const float *X = p.act, *H1 = X + P_TRAIN * PF, *H2 = H1 + P_TRAIN * PH, *Y = H2 + P_TRAIN * PH, *T = Y + P_TRAIN;
-    __shared__ float w2[PH * PH];
-    __shared__ float w3[PH];
-    __shared__ float d2[PB][PH], d1[PB][PH], h1[PB][PH], h2[PB][PH];
+    __shared__ __align__(16) float w2[PH * PH];
+    __shared__ __align__(16) float d2[PB * PR], d1[PB * PR], h1[PB * PR], h2[PB * PR];
     __shared__ float xs[PB][PF], dys[PB];
-    __shared__ float lsum[8];
-    for (int i = threadIdx.x; i < PH * PH; i += blockDim.x) w2[i] = __bfloat162float(p.w2b[i]);
-    for (int i = threadIdx.x; i < PH; i += blockDim.x) w3[i] = p.param[P_W3 + i];
-    float acc[P_PER_THREAD];
-#pragma unroll
-    for (int r = 0; r < P_PER_THREAD; ++r) acc[r] = 0.f;
-    float lacc = 0.f;
+    const uint32_t tid = threadIdx.x;
+    auto at = [](float *row, uint32_t c) { return reinterpret_cast<float4 *>(row + c); };
+    for (uint32_t i = tid; i < PH * PH / 2; i += blockDim.x) {
+        const float2 w = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162 *>(p.w2b)[i]);
+        w2[2 * i] = w.x;
+        w2[2 * i + 1] = w.y;
+    }
+    // this thread's element of a tile, its 4 x 4 block of W2, its W1 parameter
+    const uint32_t r0 = tid / 16u, c0 = tid % 16u * 4u;
+    const float4 w3 = make_float4(p.param[P_W3 + c0], p.param[P_W3 + c0 + 1], p.param[P_W3 + c0 + 2], p.param[P_W3 + c0 + 3]);
+    float acc2[4][4] = {}, acc1 = 0.f, acco = 0.f, lacc = 0.f;
     const uint32_t n_tiles = (S + PB - 1) / PB;
     for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-        const uint32_t s0 = tile * PB;
-        __syncthreads();  // w2 / w3 loaded, or the previous tile consumed
-        if (threadIdx.x < PB) {
-            const uint32_t s = s0 + threadIdx.x;
-            const float e = s < S ? Y[s] - T[s] : 0.f;
-            dys[threadIdx.x] = 2.f * e / (float)S;
+        const uint32_t s0 = tile * PB, s = s0 + r0;
+        float4 v1 = make_float4(0.f, 0.f, 0.f, 0.f), v2 = v1;
+        float e = 0.f;
+        if (s < S) {
+            v1 = *reinterpret_cast<const float4 *>(H1 + s * PH + c0);
+            v2 = *reinterpret_cast<const float4 *>(H2 + s * PH + c0);
+            e = Y[s] - T[s];
+        }
+        const float dy = 2.f * e / (float)S;
+        __syncthreads();  // w2 loaded, or the previous tile consumed
+        *at(h1 + r0 * PR, c0) = v1;
+        *at(h2 + r0 * PR, c0) = v2;
+        *at(d2 + r0 * PR, c0) = make_float4(v2.x > 0.f ? dy * w3.x : 0.f, v2.y > 0.f ? dy * w3.y : 0.f,
+                                            v2.z > 0.f ? dy * w3.z : 0.f, v2.w > 0.f ? dy * w3.w : 0.f);
+        if (c0 == 0u) {
+            dys[r0] = dy;
             lacc += e * e;
-            for (int f = 0; f < PF; ++f)  // layer 1 consumed BF16(x)
-                xs[threadIdx.x][f] = s < S ? __bfloat162float(__float2bfloat16_rn(X[s * PF + f])) : 0.f;
         }
-        for (uint32_t i = threadIdx.x; i < PB * PH; i += blockDim.x) {
-            const uint32_t r = i / PH, j = i % PH, s = s0 + r;
-            h1[r][j] = s < S ? H1[s * PH + j] : 0.f;
-            h2[r][j] = s < S ? H2[s * PH + j] : 0.f;
+        if (tid < PB * PF) {  // layer 1 consumed BF16(x)
+            const uint32_t sx = s0 + tid / PF;
+            xs[tid / PF][tid % PF] = sx < S ? __bfloat162float(__float2bfloat16_rn(X[sx * PF + tid % PF])) : 0.f;
         }
         __syncthreads();
-        for (uint32_t i = threadIdx.x; i < PB * PH; i += blockDim.x) {
-            const uint32_t r = i / PH, j = i % PH;
-            d2[r][j] = h2[r][j] > 0.f ? dys[r] * w3[j] : 0.f;
-        }
-        __syncthreads();
-        for (uint32_t i = threadIdx.x; i < PB * PH; i += blockDim.x) {
-            const uint32_t r = i / PH, k = i % PH;
-            float a = 0.f;
-#pragma unroll 16
-            for (int j = 0; j < PH; ++j) a += d2[r][j] * w2[j * PH + k];
-            d1[r][k] = h1[r][k] > 0.f ? a : 0.f;
-        }
-        __syncthreads();
+        {  // dz1 of sample r0, units c0 .. c0 + 3
+            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+            for (uint32_t j4 = 0; j4 < PH; j4 += 4) {
+                const float4 d = *at(d2 + r0 * PR, j4);
+                const float dj[4] = {d.x, d.y, d.z, d.w};
 #pragma unroll
-        for (int q = 0; q < P_PER_THREAD; ++q) {
-            const uint32_t i = threadIdx.x + 256u * q;
-            float a = 0.f;
-            if (i < (uint32_t)P_B1) {
-                const uint32_t j = i / PF, f = i % PF;
-                for (int r = 0; r < PB; ++r) a += d1[r][j] * xs[r][f];
-            } else if (i < (uint32_t)P_W2) {
-                for (int r = 0; r < PB; ++r) a += d1[r][i - P_B1];
-            } else if (i < (uint32_t)P_B2) {
-                const uint32_t j = (i - P_W2) / PH, k = (i - P_W2) % PH;
-                for (int r = 0; r < PB; ++r) a += d2[r][j] * h1[r][k];
-            } else if (i < (uint32_t)P_W3) {
-                for (int r = 0; r < PB; ++r) a += d2[r][i - P_B2];
-            } else if (i < (uint32_t)P_B3) {
-                for (int r = 0; r < PB; ++r) a += dys[r] * h2[r][i - P_W3];
-            } else if (i < (uint32_t)P_NPARAM) {
-                for (int r = 0; r < PB; ++r) a += dys[r];
+                for (uint32_t i = 0; i < 4; ++i) {
+                    const float4 w = *at(w2 + (j4 + i) * PH, c0);
+                    a.x += dj[i] * w.x;
+                    a.y += dj[i] * w.y;
+                    a.z += dj[i] * w.z;
+                    a.w += dj[i] * w.w;
+                }
             }
-            acc[q] += a;
+            *at(d1 + r0 * PR, c0) = make_float4(v1.x > 0.f ? a.x : 0.f, v1.y > 0.f ? a.y : 0.f, v1.z > 0.f ? a.z : 0.f,
+                                                v1.w > 0.f ? a.w : 0.f);
         }
+        float a2[4][4] = {};
+#pragma unroll 4
+        for (int r = 0; r < PB; ++r) {
+            const float4 d = *at(d2 + r * PR, r0 * 4u), h = *at(h1 + r * PR, c0);
+            const float dj[4] = {d.x, d.y, d.z, d.w}, hk[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int k = 0; k < 4; ++k) a2[j][k] += dj[j] * hk[k];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc2[j][k] += a2[j][k];
+        float ao = 0.f;  // b2, w3, b3
+        if (tid < PH)
+            for (int r = 0; r < PB; ++r) ao += d2[r * PR + tid];
+        else if (tid < 2 * PH)
+            for (int r = 0; r < PB; ++r) ao += dys[r] * h2[r * PR + tid - PH];
+        else if (tid == 2 * PH)
+            for (int r = 0; r < PB; ++r) ao += dys[r];
+        __syncthreads();
+        float a1 = 0.f;
+        for (int r = 0; r < PB; ++r) a1 += d1[r * PR + tid / PF] * xs[r][tid % PF];
+        acc1 += a1;
+        if (tid >= 192u)  // b1
+            for (int r = 0; r < PB; ++r) ao += d1[r * PR + tid - 192u];
+        acco += ao;
     }
 #pragma unroll
-    for (int q = 0; q < P_PER_THREAD; ++q) {
-        const uint32_t i = threadIdx.x + 256u * q;
-        if (i < (uint32_t)P_NPARAM && acc[q] != 0.f) atomicAdd(&p.grad[i], acc[q]);
-    }
-    for (int o = 16; o > 0; o >>= 1) lacc += __shfl_xor_sync(FULL, lacc, o);
-    if ((threadIdx.x & 31) == 0) lsum[threadIdx.x >> 5] = lacc;
+    for (int j = 0; j < 4; ++j)
+        atomicAdd(reinterpret_cast<float4 *>(p.grad + P_W2 + (r0 * 4u + j) * PH + c0),
+                  make_float4(acc2[j][0], acc2[j][1], acc2[j][2], acc2[j][3]));
+    atomicAdd(&p.grad[P_W1 + tid], acc1);
+    const int other = tid < PH ? P_B2 + (int)tid : tid < 2 * PH ? P_W3 + (int)tid - PH
+                      : tid == 2 * PH ? P_B3 : tid >= 192u ? P_B1 + (int)tid - 192 : -1;
+    if (other >= 0) atomicAdd(&p.grad[other], acco);
+    // the squared errors of the tiles' rows, one per 16 threads
+    lacc += __shfl_xor_sync(FULL, lacc, 16);
+    __syncthreads();  // dys is read to the end of the last tile
+    if ((tid & 31u) == 0u) dys[tid >> 5] = lacc;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
         float t = 0.f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += lsum[w];
+        for (int w = 0; w < 8; ++w) t += dys[w];
         atomicAdd(&p.loss[1], t);
     }
 }
+static_assert(P_W2 % 4 == 0 && PH == 64 && PF == 4, "the layout of a thread's parameters");
 
 // Adam (Kingma & Ba, 2015) on the FP32 master parameters; each updated weight
 // of W1 / W2 is also written to its BF16 copy (the zero padding of W1's K
@@ -356,68 +396,62 @@ __global__ void pred_roll(PredDev p, uint32_t *__restrict__ counts) {
     }
 }
 
-// Top-k scores -> staged set, in one block of 1024 threads.  Each score becomes
-// a 16-bit order-preserving key (sign, exponent and 7 mantissa bits) kept in
-// shared memory, so the passes below read no global memory: two 256-bin
-// histogram passes find the k-th largest key (one shared atomic per distinct
-// bin of a warp); buckets above it are taken, then ties in bucket order until
-// k.  Thread t owns buckets 64t .. 64t+63 (its bitmap words 2t, 2t+1); their
-// keys are row t of the shared array, rows padded by 4 bytes so that the
-// warp's row walks hit 32 different banks.  Outputs: the bitmap and per-word
-// ranks and the bucket -> group map.  The first thread also ends the
-// predictor step (training step count when `trained`, batches seen).
-constexpr uint32_t SELECT_ROW = 66u;  // 64 keys + 2 of padding
-constexpr uint32_t SELECT_SMEM = STAGE_BUCKETS / 64u * SELECT_ROW * 2u;
-__device__ __forceinline__ uint32_t select_idx(uint32_t b) { return (b >> 6) * SELECT_ROW + (b & 63u); }
+// Top-k scores -> staged set, in one cluster of eight blocks of 1024 threads,
+// eight buckets to a thread.  Each score becomes a 16-bit order-preserving key
+// (sign, exponent and 7 mantissa bits) in a register: two 256-bin histogram
+// passes find the k-th largest key (one shared atomic per distinct bin of a
+// warp; the blocks read one another's histograms); buckets above it are taken,
+// then ties in bucket order until k.  Outputs: the bitmap and per-word ranks
+// and the bucket -> group map.  The first thread also ends the predictor step
+// (training step count when `trained`, batches seen).  (One block of 64 buckets
+// to a thread, its keys in shared memory: 45 to 72 us; the cluster: 10 to 15.)
+constexpr uint32_t SEL_BLOCKS = 8u;
+static_assert(SEL_BLOCKS * 1024u * 8u == STAGE_BUCKETS, "eight buckets to a thread");
 
-__global__ void __launch_bounds__(1024) pred_select(PredDev p, uint32_t k, uint32_t *__restrict__ bits,
-                                                    uint32_t *__restrict__ rank, uint16_t *__restrict__ map,
-                                                    int trained) {
-    extern __shared__ __align__(16) uint16_t keys[];  // STAGE_BUCKETS / 64 rows of SELECT_ROW
-    __shared__ uint32_t hist[256];
-    __shared__ uint32_t sel_bin, sel_rem;
+__global__ void __cluster_dims__(SEL_BLOCKS, 1, 1) __launch_bounds__(1024)
+    pred_select(PredDev p, uint32_t k, uint32_t *__restrict__ bits, uint32_t *__restrict__ rank,
+                uint16_t *__restrict__ map, int trained) {
+    __shared__ uint32_t hist[2][256], all[256];
+    __shared__ uint32_t sel_bin, sel_rem, total;
     __shared__ uint32_t wsum[32];
-    const uint32_t tid = threadIdx.x;
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, me = cluster.block_rank();
+    const uint32_t b0 = (me * 1024u + tid) * 8u;
     auto okey16 = [](float f) {
         const uint32_t u = __float_as_uint(f);
-        return (uint16_t)(((u & 0x80000000u) ? ~u : (u | 0x80000000u)) >> 16);
+        return ((u & 0x80000000u) ? ~u : (u | 0x80000000u)) >> 16;
     };
-    // keys of all buckets, loaded 16 bytes a thread, consecutive threads on
-    // consecutive buckets
-    const float4 *src = reinterpret_cast<const float4 *>(p.scores);
-#pragma unroll 4
-    for (uint32_t v = tid; v < STAGE_BUCKETS / 4u; v += blockDim.x) {
-        const float4 f = src[v];
-        uint16_t *k4 = keys + select_idx(4u * v);  // four buckets of one row
-        k4[0] = okey16(f.x);
-        k4[1] = okey16(f.y);
-        k4[2] = okey16(f.z);
-        k4[3] = okey16(f.w);
-    }
+    const float4 f0 = reinterpret_cast<const float4 *>(p.scores + b0)[0],
+                 f1 = reinterpret_cast<const float4 *>(p.scores + b0)[1];
+    const uint32_t key[8] = {okey16(f0.x), okey16(f0.y), okey16(f0.z), okey16(f0.w),
+                             okey16(f1.x), okey16(f1.y), okey16(f1.z), okey16(f1.w)};
+    if (tid < 256u) hist[0][tid] = hist[1][tid] = 0u;
+    __syncthreads();
     // two passes: the high byte of the k-th largest key, then its low byte
     uint32_t hi = 0, remaining = k;
     for (int pass = 0; pass < 2; ++pass) {
-        if (tid < 256) hist[tid] = 0;
-        __syncthreads();
-        for (uint32_t b = tid; b < STAGE_BUCKETS; b += blockDim.x) {  // interleaved
-            const uint32_t u = keys[select_idx(b)];
-            const bool in = pass == 0 || (u >> 8) == hi;
-            const uint32_t bin = !in ? 256u : pass == 0 ? (u >> 8) : (u & 255u);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const bool in = pass == 0 || (key[i] >> 8) == hi;
+            const uint32_t bin = !in ? 256u : pass == 0 ? key[i] >> 8 : key[i] & 255u;
             const unsigned peers = __match_any_sync(FULL, bin);
-            if (in && (tid & 31u) == (uint32_t)__ffs(peers) - 1u) atomicAdd(&hist[bin], (uint32_t)__popc(peers));
+            if (in && lane == (uint32_t)__ffs(peers) - 1u) atomicAdd(&hist[pass][bin], (uint32_t)__popc(peers));
+        }
+        cluster.sync();
+        if (tid < 256u) {
+            uint32_t sum = 0;
+#pragma unroll
+            for (uint32_t r = 0; r < SEL_BLOCKS; ++r) sum += *cluster.map_shared_rank(&hist[pass][tid], r);
+            all[tid] = sum;
         }
         __syncthreads();
         if (tid < 32) {  // the bin holding the remaining-th largest key: warp-wide suffix sums
             const uint32_t lo = (31u - tid) * 8u;  // lane 0 holds the highest bins
             uint32_t c[8], tot = 0;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) tot += (c[i] = hist[lo + i]);
-            uint32_t incl = tot;  // keys in this lane's bins and all higher ones
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t v = __shfl_up_sync(FULL, incl, o);
-                if (tid >= (uint32_t)o) incl += v;
-            }
-            const uint32_t above = incl - tot;  // keys in higher lanes' bins
+            for (int i = 0; i < 8; ++i) tot += (c[i] = all[lo + i]);
+            const uint32_t incl = (uint32_t)warp_incl_scan((int)tot);  // keys in this lane's bins and all higher ones
+            const uint32_t above = incl - tot;                        // keys in higher lanes' bins
             if (above < remaining && incl >= remaining) {
                 uint32_t acc = above, bin = lo;
                 for (int i = 7; i >= 0; --i) {
@@ -436,77 +470,53 @@ __global__ void __launch_bounds__(1024) pred_select(PredDev p, uint32_t k, uint3
         remaining = sel_rem;
     }
     // hi: the k-th largest key; `remaining` of the buckets with that key are
-    // still needed, taken in bucket order (exclusive scan of each thread's
-    // count of such buckets among its 64)
-    uint32_t tie_before = 0;
-    {
-        uint32_t mine = 0;
-        for (uint32_t i = 0; i < 64; ++i) mine += keys[tid * SELECT_ROW + i] == hi;
-        uint32_t incl = mine;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(FULL, incl, o);
-            if ((tid & 31) >= (uint32_t)o) incl += v;
-        }
-        if ((tid & 31) == 31) wsum[tid >> 5] = incl;
-        __syncthreads();
-        if (tid < 32) {
-            uint32_t w = wsum[tid], wi = w;
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t v = __shfl_up_sync(FULL, wi, o);
-                if (tid >= (uint32_t)o) wi += v;
-            }
-            wsum[tid] = wi - w;
-        }
-        __syncthreads();
-        tie_before = wsum[tid >> 5] + incl - mine;
-    }
-    // bitmap words: thread owns buckets tid*64 .. tid*64+63 = words 2 tid, 2 tid + 1
-    uint32_t word[2] = {0u, 0u};
-    for (uint32_t i = 0; i < 64; ++i) {
-        const uint32_t u = keys[tid * SELECT_ROW + i];
-        bool take = u > hi;
-        if (u == hi) {
-            take = tie_before < remaining;
-            ++tie_before;
-        }
-        if (take) word[i >> 5] |= 1u << (i & 31u);
-    }
-    bits[2 * tid] = word[0];
-    bits[2 * tid + 1] = word[1];
-    // rank: exclusive scan of popcounts over the 2048 words
-    const uint32_t c0 = __popc(word[0]), mine = c0 + __popc(word[1]);
-    uint32_t incl = mine;
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(FULL, incl, o);
-        if ((tid & 31) >= (uint32_t)o) incl += v;
-    }
-    __syncthreads();
-    if ((tid & 31) == 31) wsum[tid >> 5] = incl;
+    // still needed, taken in bucket order.  Scan of (taken outright << 16 | ties)
+    // over the block's threads, then the blocks before.
+    uint32_t mine = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) mine += key[i] > hi ? 0x10000u : key[i] == hi ? 1u : 0u;
+    const uint32_t incl = (uint32_t)warp_incl_scan((int)mine);
+    if (lane == 31u) wsum[tid >> 5] = incl;
     __syncthreads();
     if (tid < 32) {
-        uint32_t w = wsum[tid], wi = w;
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(FULL, wi, o);
-            if (tid >= (uint32_t)o) wi += v;
-        }
+        const uint32_t w = wsum[tid], wi = (uint32_t)warp_incl_scan((int)w);
         wsum[tid] = wi - w;
+        if (tid == 31) total = wi;
     }
-    __syncthreads();
-    const uint32_t r0 = wsum[tid >> 5] + incl - mine;
-    rank[2 * tid] = r0;
-    rank[2 * tid + 1] = r0 + c0;
-    // the map, row by row into the keys' place, then out in bucket order
-    uint32_t r = r0;
-    for (uint32_t i = 0; i < 64; ++i) {
-        const bool on = (word[i >> 5] >> (i & 31u)) & 1u;
-        keys[tid * SELECT_ROW + i] = on ? (uint16_t)r++ : (uint16_t)STAGE_NONE;
+    cluster.sync();
+    uint32_t gt = 0, ties = 0;  // of the buckets before this thread's
+#pragma unroll
+    for (uint32_t r = 0; r < SEL_BLOCKS; ++r) {
+        const uint32_t t = r < me ? *cluster.map_shared_rank(&total, r) : 0u;
+        gt += t >> 16;
+        ties += t & 0xFFFFu;
     }
-    __syncthreads();
-    for (uint32_t b = tid; b < STAGE_BUCKETS; b += blockDim.x) map[b] = keys[select_idx(b)];
-    if (tid == 0) {
+    const uint32_t before = wsum[tid >> 5] + incl - mine;
+    gt += before >> 16;
+    ties += before & 0xFFFFu;
+    const uint32_t r0 = gt + min(ties, remaining);
+    uint32_t group = r0, mask = 0, m[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const bool take = key[i] > hi || (key[i] == hi && ties++ < remaining);
+        mask |= take ? 1u << i : 0u;
+        m[i] = take ? group++ : STAGE_NONE;
+    }
+    reinterpret_cast<uint4 *>(map + b0)[0] =
+        make_uint4(m[0] | m[1] << 16, m[2] | m[3] << 16, m[4] | m[5] << 16, m[6] | m[7] << 16);
+    // a bitmap word is four threads'
+    uint32_t word = mask << (8u * (tid & 3u));
+    word |= __shfl_xor_sync(FULL, word, 1);
+    word |= __shfl_xor_sync(FULL, word, 2);
+    if ((tid & 3u) == 0u) {
+        bits[b0 >> 5] = word;
+        rank[b0 >> 5] = r0;
+    }
+    if (b0 == 0u) {
         if (trained) p.state[1] += 1;
         p.state[2] += 1;
     }
+    cluster.sync();  // no block leaves while another reads its shared memory
 }
 
 }  // namespace ltpg
@@ -582,7 +592,6 @@ int ltpg_predictor_enable(ltpg_ctx *c, const ltpg_predictor_cfg *cfg) {
         PCK(cudaMalloc(&d.act, (size_t)P_TRAIN * (PF + 2 * PH + 2) * 4));
         PCK(cudaMalloc(&d.state, 16));
         PCK(cudaMalloc(&d.loss, 8));
-        PCK(cudaFuncSetAttribute(pred_select, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SELECT_SMEM));
         PCK(cudaMalloc(&P->io, (size_t)P_TRAIN * 8 * 4));
     }
     ltpg_predictor_state *P = c->pred;
@@ -675,17 +684,17 @@ cudaError_t predictor_after_batch(ltpg_ctx *c) {
     count_launch(c);
     int trained = 0;
     if (c->pred_train) {
-        pred_forward<<<64, 256, 0, c->stream>>>(P->d, P_TRAIN, 1, nullptr, nullptr);
-        pred_backward<<<64, 256, 0, c->stream>>>(P->d, P_TRAIN);
+        pred_forward<<<P_TRAIN / 32, 64, 0, c->stream>>>(P->d, P_TRAIN, 1, nullptr, nullptr);
+        pred_backward<<<128, 256, 0, c->stream>>>(P->d, P_TRAIN);
         pred_adam<<<18, 256, 0, c->stream>>>(P->d, P->lr, P_TRAIN);
         count_launch(c, 3);
         trained = 1;
     }
-    pred_forward<<<c->sm_count, 256, 0, c->stream>>>(P->d, STAGE_BUCKETS, 0, nullptr, nullptr);
+    pred_forward<<<STAGE_BUCKETS / 128, 256, 0, c->stream>>>(P->d, STAGE_BUCKETS, 0, nullptr, nullptr);
     count_launch(c);
     if (c->stage_on) {
         const uint32_t ways = c->launch_y.ways ? c->launch_y.ways : 4u;
-        pred_select<<<1, 1024, SELECT_SMEM, c->stream>>>(P->d, STAGE_MAX_ENTRIES / ways, c->stage_bits,
+        pred_select<<<SEL_BLOCKS, 1024, 0, c->stream>>>(P->d, STAGE_MAX_ENTRIES / ways, c->stage_bits,
                                                          c->stage_rank, c->stage_map, trained);
     } else {
         pred_step_done<<<1, 32, 0, c->stream>>>(P->d, trained);
