@@ -117,13 +117,6 @@ __device__ __forceinline__ void write_txn_updates(const YcsbTunedArgs &a, uint32
     }
 }
 
-// Late reads of one tile whose commit flags are in fl: the lpt lanes of a
-// transaction (a power of two, aligned in the warp) take one op each; the
-// point reads of committed transactions are gathered five lanes to a row (one
-// 16-byte chunk each, six rows per round), a range scan by the whole warp over
-// its contiguous rows.  results[t] = sum over reads of xor(row) * (2j + 1), as
-// at execute; 0 for an aborted transaction.  No row is written before the
-// next kernel, so every read sees the batch-start image.
 // Row gather of a warp: the rows of up to 32 keys, five lanes to a row (one
 // 16-byte chunk each, six rows per round on lanes 0..29), so a row costs one or
 // two cache-line requests.  `need` (a ballot) names the lanes that want a row;
@@ -227,6 +220,56 @@ __device__ __forceinline__ unsigned long long rows_fold_shfl(unsigned need, cons
     return x;
 }
 
+// The xor of the rows of each lane's scan in `scans` (the other lanes keep x):
+// eight lanes to a scan, four scans at a time, each lane loading the 16-byte
+// chunks of its place in the 128-byte lines that the scan's rows cover, four
+// lines in flight.  Instructions bound it: a whole warp to a scan folded five
+// levels of shuffles for two loads, and waited for them before the next scan's
+// (2^18 x 10 scans of 10 keys at theta 0.99: 291 -> 153 us).
+__device__ __forceinline__ unsigned long long scans_fold(const YcsbTunedArgs &a, RowScratch *ws, uint32_t w,
+                                                         unsigned scans, unsigned long long x) {
+    const uint32_t lane = threadIdx.x & 31, l = lane & 7u, n = __popc(scans);
+    const uint32_t rank = __popc(scans & ((1u << lane) - 1u));
+    const bool own = (scans >> lane) & 1u;
+    const uint32_t key = ycsb_key(w);
+    __syncwarp();  // the point reads' fold is over
+    if (own) ws->key[rank] = key | ((uint32_t)scan_last(w, a.n) - key) << LTPG_YCSB_KEY_BITS;
+    __syncwarp();
+    for (uint32_t base = 0; base < n; base += 4u) {
+        const uint32_t i = base + (lane >> 3);
+        unsigned long long c = 0;
+        if (i < n) {
+            const uint32_t e = ws->key[i];
+            const uint64_t first = (uint64_t)(e & ((1u << LTPG_YCSB_KEY_BITS) - 1u)) * 5u;  // in chunks of the table
+            const uint32_t off = (uint32_t)first & 7u, end = off + ((e >> LTPG_YCSB_KEY_BITS) + 1u) * 5u;
+            const ulonglong2 *p = reinterpret_cast<const ulonglong2 *>(a.rows) + (first - off);
+            for (uint32_t q = l; q < end; q += 32u) {
+                ulonglong2 v[4];
+#pragma unroll
+                for (uint32_t r = 0; r < 4; ++r) {
+                    const uint32_t at = q + 8u * r;
+                    v[r] = at >= off && at < end ? ld_nc16_issue(p + at) : make_ulonglong2(0ull, 0ull);
+                }
+#pragma unroll
+                for (uint32_t r = 0; r < 4; ++r) c ^= v[r].x ^ v[r].y;
+            }
+        }
+#pragma unroll
+        for (uint32_t o = 4; o >= 1u; o >>= 1) c ^= __shfl_xor_sync(FULL, c, o);
+        if (l == 0u && i < n) ws->part[i] = c;
+    }
+    __syncwarp();
+    return own ? ws->part[rank] : x;
+}
+
+// Late reads of one tile whose commit flags are in fl: the lpt lanes of a
+// transaction (a power of two, aligned in the warp) take one op each; the
+// point reads of committed transactions are gathered five lanes to a row (one
+// 16-byte chunk each, six rows per round), range scans eight
+// lanes to a scan.  results[t] = sum over reads of xor(row) * (2j + 1), as
+// at execute; 0 for an aborted transaction.  No row is written before the
+// next kernel, so every read sees the batch-start image.
+//
 // One step of the lanes of a warp (all 32 call it): lane j of transaction t
 // (own: the lane holds an op slot of a transaction; com: t committed).
 __device__ __forceinline__ void late_read_step(const YcsbTunedArgs &a, RowScratch *ws, uint32_t t, uint32_t j,
@@ -245,20 +288,8 @@ __device__ __forceinline__ void late_read_step(const YcsbTunedArgs &a, RowScratc
             rows_issue(a.rows, ws, key, need, ch);
             x = rows_fold(ws, need, ch);
         }
-        const uint32_t last = scan ? (uint32_t)scan_last(w, a.n) : 0u;
-        for (unsigned m = __ballot_sync(FULL, scan); m; m &= m - 1u) {
-            const uint32_t src = (uint32_t)__ffs(m) - 1u;
-            const uint32_t k0 = __shfl_sync(FULL, key, src), k1 = __shfl_sync(FULL, last, src);
-            const uint32_t chunks = (k1 - k0 + 1u) * 5u;
-            const ulonglong2 *p = reinterpret_cast<const ulonglong2 *>(a.rows + (uint64_t)k0 * LTPG_YCSB_FIELDS);
-            unsigned long long c_all = 0;
-            for (uint32_t c = lane; c < chunks; c += 32u) {
-                const ulonglong2 q = ld_nc16(p + c);
-                c_all ^= q.x ^ q.y;
-            }
-            for (uint32_t o = 16; o >= 1u; o >>= 1) c_all ^= __shfl_xor_sync(FULL, c_all, o);
-            if (lane == src) x = c_all;
-        }
+        const unsigned scans = __ballot_sync(FULL, scan);
+        if (scans) x = scans_fold(a, ws, w, scans, x);  // warp-uniform
         unsigned long long part = rd ? x * (2ull * j + 1ull) : 0ull;
         for (uint32_t o = lpt >> 1; o >= 1; o >>= 1) part += __shfl_xor_sync(FULL, part, o);
         if (own && j == 0u) a.results[t] = (int64_t)part;
@@ -297,11 +328,12 @@ __device__ __forceinline__ void late_read_loop(const YcsbTunedArgs &a, RowScratc
 
 // The grid-stride kernels below are instantiated per block size (BS = 128,
 // 256, 512: launch setting block_threads), each with launch bounds of its own
-// block: bounds above the block change the compiler's register choice (the
-// read kernel takes 58 registers under 512-thread bounds against 40 under
-// 256, and loses a third of its resident warps).
+// block: bounds above the block change the compiler's register choice.  The
+// read kernel is held to 1,280 threads an SM (48 registers): left alone it took
+// 32 and waited for each pair of rows (2^20 x 16 at theta 0.99 172 us against
+// 169, scans 170 against 153); for 1,536 threads (40) 179 and 145.
 template <int BS>
-__global__ void __launch_bounds__(BS) ycsb_read_late(YcsbTunedArgs a) {
+__global__ void __launch_bounds__(BS, 1280 / BS) ycsb_read_late(YcsbTunedArgs a) {
     late_read_loop<false>(a, row_scratch<BS>());
 }
 
