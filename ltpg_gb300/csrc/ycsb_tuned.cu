@@ -376,24 +376,29 @@ __device__ __forceinline__ void wf_register_writes(const YcsbTunedArgs &a, uint6
         const uint4 w4 = ld_nc_u4(vp + v);
         const uint32_t t = v / vpt;
         const uint32_t words[4] = {w4.x, w4.y, w4.z, w4.w};
+        // the looks at the slots and the bitmap of a vector are in flight together:
+        // most warps hold an update, and one after another they were this pass
+        // (2^20 x 16, 5 % updates: 36 -> 27 us; 50 -> 34 at theta 0)
+        bool upd[4];
+        uint64_t cur[4];
+        uint32_t seen[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const uint32_t w = words[q];
-            if (ycsb_is_pad(w)) continue;
-            const uint32_t key = ycsb_key(w);
-            if (key >= a.n) {
-                report_error(a.ctl, DERR_BOUNDS, t);
-                continue;
-            }
-            if (!ycsb_is_update(w)) continue;
-            unsigned long long *slot = &a.reg[key].w;
+            const uint32_t w = words[q], key = ycsb_key(w);
+            upd[q] = !ycsb_is_pad(w) && ycsb_is_update(w) && key < a.n;
+            if (!ycsb_is_pad(w) && key >= a.n) report_error(a.ctl, DERR_BOUNDS, t);
+            cur[q] = upd[q] && a.filter ? ld_filter_u64<kCoh>(&a.reg[key].w) : ~0ull;
+            unsigned *bw = a.wbits + (key >> 5);
+            seen[q] = !upd[q] ? ~0u : kCoh ? ld_gpu_u32(bw) : ld_ca_u32(bw);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t key = ycsb_key(words[q]);
             const unsigned long long mine = tag | t;
-            if (!a.filter || ld_filter_u64<kCoh>(slot) > mine) red_min(slot, mine);
+            if (upd[q] && cur[q] > mine) red_min(&a.reg[key].w, mine);
             // bits are only set within a batch: a bit seen set needs no atomic
             // (hot keys' updates would otherwise all hit one word)
-            unsigned *bw = a.wbits + (key >> 5);
-            const uint32_t seen = kCoh ? ld_gpu_u32(bw) : ld_ca_u32(bw);
-            if (!((seen >> (key & 31u)) & 1u)) atomicOr(bw, 1u << (key & 31u));
+            if (!((seen[q] >> (key & 31u)) & 1u)) atomicOr(a.wbits + (key >> 5), 1u << (key & 31u));
         }
     }
 }
@@ -489,14 +494,14 @@ __device__ __forceinline__ void wf_list_updates(const YcsbTunedArgs &a, bool act
 // with a writer; the RAW bit is OR-ed into the transaction's flag byte
 // (zeroed by (1)) with a 32-bit atomic.
 // kList: the pass also writes the update list (wf_list_updates); its stores
-// wait behind the slot loads this pass is bound by.
+// wait behind the slot loads this pass is bound by.  Transactions t0 .. t1 - 1.
 template <bool kCoh, bool kList = false>
-__device__ __forceinline__ void wf_register_reads(const YcsbTunedArgs &a, uint32_t epoch) {
-    const uint32_t vpt = a.stride / 4u, nvec = a.B * vpt;
+__device__ __forceinline__ void wf_register_reads(const YcsbTunedArgs &a, uint32_t epoch, uint32_t t0, uint32_t t1) {
+    const uint32_t vpt = a.stride / 4u, nvec = t1 * vpt;
     const uint32_t step = gridDim.x * blockDim.x;
     const uint4 *vp = reinterpret_cast<const uint4 *>(a.ops);
     // a block-uniform loop, so that whole warps reach the warp-wide calls below
-    for (uint32_t base = blockIdx.x * blockDim.x; base < nvec; base += step) {
+    for (uint32_t base = t0 * vpt + blockIdx.x * blockDim.x; base < nvec; base += step) {
         const uint32_t v = base + threadIdx.x;
         const bool act = v < nvec;
         const uint4 w4 = act ? ld_nc_u4(vp + v)
@@ -542,8 +547,8 @@ __global__ void __launch_bounds__(BS) ycsb_wf_writes(YcsbTunedArgs a) {
 
 // ---- write-first with the update list (stride / 4 a power of two <= 8) --------
 template <int BS>
-__global__ void __launch_bounds__(BS) ycsb_wf_reads_list(YcsbTunedArgs a) {
-    wf_register_reads<false, true>(a, a.ctl->epoch);
+__global__ void __launch_bounds__(BS) ycsb_wf_reads_list(YcsbTunedArgs a, uint32_t t0, uint32_t t1) {
+    wf_register_reads<false, true>(a, a.ctl->epoch, t0, t1);
 }
 
 // Entries of the batch's update list: val_off[B], bounded by the list.
@@ -1217,7 +1222,7 @@ __device__ __forceinline__ void ycsb_persistent_body(const YcsbTunedArgs &a) {
     if (kLate && !kStage && a.late == 3u) {  // write-first: five phases, four grid barriers
         wf_register_writes<true>(a, tag);
         bool ok = grid_barrier(a.ctl);
-        if (ok) wf_register_reads<true, true>(a, epoch);
+        if (ok) wf_register_reads<true, true>(a, epoch, 0u, a.B);
         ok = ok && grid_barrier(a.ctl);
         if (ok) wf_check_list<true>(a, epoch);
         ok = ok && grid_barrier(a.ctl);
@@ -1403,7 +1408,21 @@ static cudaError_t launch_write_first_t(ltpg_ctx *c, const YcsbTunedArgs &a) {
     prof_mark(c, 0);
     count_launch(c, 2);
     ycsb_wf_writes<BS><<<stride_grid(c, (const void *)ycsb_wf_writes<BS>, nvec), BS, 0, c->stream>>>(a);
-    ycsb_wf_reads_list<BS><<<stride_grid(c, (const void *)ycsb_wf_reads_list<BS>, nvec), BS, 0, c->stream>>>(a);
+    // The smallest TIDs register first, in a launch of their own: a wave finds
+    // every slot empty, so all reads of a hot key were sent and queued at its
+    // slot, where now the filter knows the least TID of every key read in the
+    // head (theta 0.99: 2^20 x 16 145 -> 123 us, 65,536 x 16 41 -> 22; a head of
+    // 4,096 or 16,384 no better).  With the filter only, which says that keys
+    // are hot, and from 8,192 transactions on: else the launch costs more (theta
+    // 0: 2^20 x 16 125 -> 129 us, 65,536 x 16 16 -> 20).
+    const uint32_t head = a.filter && a.B >= 8192u ? 1024u : 0u;
+    if (head) {
+        count_launch(c);
+        ycsb_wf_reads_list<BS><<<stride_grid(c, (const void *)ycsb_wf_reads_list<BS>, (uint64_t)head * a.stride / 4),
+                                 BS, 0, c->stream>>>(a, 0u, head);
+    }
+    ycsb_wf_reads_list<BS>
+        <<<stride_grid(c, (const void *)ycsb_wf_reads_list<BS>, nvec), BS, 0, c->stream>>>(a, head, a.B);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     prof_mark(c, 1);
