@@ -260,11 +260,9 @@ def profile_traffic(workload, kernel):
 def ycsb_exec_kernel_name(launch, stride):
     """Name of the execute kernel the tuned path launches for this shape."""
     opt = (launch or {}).get("ops_per_thread", 1)
-    if (opt == 1 or (launch or {}).get("late_reads")) and stride <= 32:
-        return "ycsb_exec_coop"
-    if opt in (2, 4) and stride % opt == 0 and ((stride // opt) & (stride // opt - 1)) == 0:
+    if not (launch or {}).get("late_reads") and opt in (2, 4) and ((stride // opt) & (stride // opt - 1)) == 0:
         return "ycsb_exec_fast"
-    return "ycsb_exec_tuned"
+    return "ycsb_exec_coop"
 
 
 def measured_peaks():
@@ -806,16 +804,18 @@ def bench_config(w, theta):
 
 def tpcc_registrations_per_txn(batches):
     """Registration atomics per transaction that the tuned TPC-C execute
-    kernel issues before its slot filter: NewOrder 3 header ops + 2 per order
-    line (stock write, ORDER-LINE insert), Payment 3 (customer read and write,
-    HISTORY insert); reads of WAREHOUSE / DISTRICT / ITEM do not register."""
+    kernel issues before its slot filter in a large batch without order reads:
+    NewOrder 1 (customer read) + 1 per order line (stock write), Payment 2
+    (customer read and write); inserted rows are bits of a bitmap (1 to 4 words
+    a transaction, not counted), reads of WAREHOUSE / DISTRICT / ITEM do not
+    register."""
     from ltpg_gb300 import abi
     total, n = 0, 0
     for b in batches:
         kind = b.txns["kind_info"] & 0xFF
         cnt = (b.txns["kind_info"] >> 8) & 0xFF
         no = kind == abi.TPCC_NEWORDER
-        total += int((3 + 2 * cnt[no].astype(np.int64)).sum()) + 3 * int((kind == abi.TPCC_PAYMENT).sum())
+        total += int((1 + cnt[no].astype(np.int64)).sum()) + 2 * int((kind == abi.TPCC_PAYMENT).sum())
         n += len(kind)
     return total / n
 

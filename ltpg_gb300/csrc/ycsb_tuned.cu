@@ -2,18 +2,19 @@
 //
 // Same protocol and outputs as the plain path (ycsb.cu); only the schedule
 // changes:
-//   * execute+register walks block tiles of whole transactions, reading four op
-//     words per thread with one 128-bit load;
+//   * execute+register takes one op per lane, the rows read five lanes to a row
+//     (or two or four ops per thread);
 //   * a registration goes (a) to a shared-memory staging entry when the
-//     predictor marked its key's bucket hot, else (b) through a warp-level
-//     dedupe (__match_any_sync: only the smallest TID of each key in the warp
-//     issues), then (c) an L1 read of the slot skips the atomic when the slot
-//     already holds a smaller value.  Slot values only decrease (newer batch
-//     tags are smaller, and within a batch atomicMin only lowers), so any value
-//     observed, stale or not, is >= the current one: the skip is exact;
+//     predictor marked its key's bucket hot, else (b) through a dedupe (only
+//     the smallest TID of each key in the block or the warp issues: batches of
+//     a few waves, or a launch setting), then (c) an L1 read of the slot skips
+//     the atomic when the slot already holds a smaller value.  Slot values only
+//     decrease (newer batch tags are smaller, and within a batch atomicMin only
+//     lowers), so any value observed, stale or not, is >= the current one: the
+//     skip is exact;
 //   * check and write-back run in one kernel: the commit decision of a tile is
-//     made in shared memory, then each committed transaction's thread stores
-//     its updates in op order;
+//     made in shared memory, then the threads that hold a committed
+//     transaction's op vectors store its updates, in op order;
 //   * late reads (a launch setting): execute only registers, the check kernel
 //     reads the rows of the committed transactions after the tile's commit
 //     decision, and a third kernel stores the updates, so that no aborted

@@ -100,7 +100,7 @@ def candidates(workload, staging=False, blocks=BLOCKS):
             out += [dict(block_threads=bs, ops_per_thread=1, blocks_per_sm=cap(b, bs), filter=f, dedupe=0,
                          stage_ways=4, late_reads=3) for b, f in itertools.product([0, 2, 4], [0, 1])]
         return out
-    # TPC-C: blocks of 2P threads on tiles of P transactions
+    # TPC-C: blocks on tiles of up to as many transactions as threads
     return [dict(block_threads=bs, ops_per_thread=4, blocks_per_sm=cap(b, bs), filter=f, dedupe=d, stage_ways=4,
                  late_reads=0)
             for bs in blocks for b, f, d in itertools.product([0, 2, 4, 6], [0, 1], [0, 1])]
