@@ -195,9 +195,9 @@ __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontr
 // In the kernel before it, whose blocks are all resident by then.
 __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;"); }
 
-template <class A>
-static cudaError_t launch_next(void (*k)(A), bool overlap, uint32_t grid, uint32_t threads, size_t smem,
-                               cudaStream_t st, const A &arg) {
+template <class... P, class... A>
+static cudaError_t launch_next(void (*k)(P...), bool overlap, uint32_t grid, uint32_t threads, size_t smem,
+                               cudaStream_t st, const A &...args) {
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
@@ -208,7 +208,7 @@ static cudaError_t launch_next(void (*k)(A), bool overlap, uint32_t grid, uint32
     cfg.stream = st;
     cfg.attrs = &attr;
     cfg.numAttrs = overlap ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k, arg);
+    return cudaLaunchKernelEx(&cfg, k, P(args)...);
 }
 
 __device__ __forceinline__ int warp_incl_scan(int v) {

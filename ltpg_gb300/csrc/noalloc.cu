@@ -17,21 +17,18 @@
 // the library holds this memory until the process exits.
 #include <mutex>
 
-#include "engine.h"
+#include "devutil.cuh"
 
 namespace ltpg {
 // The plain YCSB kernels (ycsb.cu), launched here on the static scratch.
 __global__ void ycsb_exec_plain(const uint32_t *__restrict__ ops, uint32_t B, uint32_t k, uint32_t stride,
                                 uint32_t tile, const uint64_t *__restrict__ rows, uint64_t n,
                                 RegSlot *__restrict__ reg, int64_t *__restrict__ results, DevCtl *ctl);
-__global__ void ycsb_check_plain(const uint32_t *__restrict__ ops, uint32_t B, uint32_t k, uint32_t stride,
-                                 uint32_t tile, const RegSlot *__restrict__ reg, uint64_t n,
-                                 uint8_t *__restrict__ flags, DevCtl *ctl);
-__global__ void ycsb_writeback_plain(const uint8_t *__restrict__ flags, uint32_t B, const uint32_t *__restrict__ ops,
-                                     uint32_t k, uint32_t stride, const uint32_t *__restrict__ val_off,
-                                     const uint64_t *__restrict__ vals, uint64_t vals_cap,
-                                     uint64_t *__restrict__ rows, uint64_t n,
-                                     uint32_t *__restrict__ bitmap, DevStats *st, DevCtl *ctl);
+__global__ void ycsb_check_write_plain(const uint32_t *__restrict__ ops, uint32_t B, uint32_t k, uint32_t stride,
+                                       const RegSlot *reg, const uint32_t *__restrict__ val_off,
+                                       const uint64_t *__restrict__ vals, uint64_t *__restrict__ rows, uint64_t n,
+                                       uint8_t *__restrict__ flags, uint32_t *__restrict__ bitmap, DevStats *st,
+                                       DevCtl *ctl);
 }  // namespace ltpg
 
 using namespace ltpg;
@@ -41,7 +38,7 @@ using namespace ltpg;
 // cleared state only when the epoch would pass its last value).
 static __device__ __align__(256) RegSlot g_noalloc_reg[LTPG_NOALLOC_MAX_RECORDS];
 // Control block (epoch, error word, completion counter), and the batch
-// counters the write-back kernel accumulates (not reported by this path).
+// counters the last kernel accumulates (not reported by this path).
 static __device__ __align__(256) DevCtl g_noalloc_ctl;
 static __device__ __align__(256) DevStats g_noalloc_stats;
 
@@ -120,11 +117,13 @@ extern "C" int ltpg_ycsb_batch_noalloc(int device, uint64_t *rows, uint64_t n_re
     // never match) except when the epoch would pass its last value
     if ((r = reserve_epoch(d, s)) != LTPG_OK) return r;
     ycsb_exec_plain<<<grid, tile * k, 0, s>>>(ops, n_txn, k, stride, tile, rows, n_records, d->reg, results, d->ctl);
-    ycsb_check_plain<<<grid, tile * k, 0, s>>>(ops, n_txn, k, stride, tile, d->reg, n_records, flags, d->ctl);
-    // the caller's vals hold val_off[n_txn] values, the bound the kernel reads
-    ycsb_writeback_plain<<<(n_txn + 255) / 256, 256, 0, s>>>(flags, n_txn, ops, k, stride, val_off, vals, ~0ull,
-                                                             rows, n_records, bitmap, d->stats, d->ctl);
     if (cudaGetLastError() != cudaSuccess) return LTPG_ERR_CUDA;
+    // the caller's vals hold val_off[n_txn] values, the bound the kernel reads;
+    // up to a few waves its launch overlaps the execute kernel
+    if (launch_next(ycsb_check_write_plain, (uint64_t)n_txn * k <= (1u << 20), (n_txn + 31) / 32, 32 * k, 0, s, ops,
+                    n_txn, k, stride, d->reg, val_off, vals, rows, n_records, flags, bitmap, d->stats,
+                    d->ctl) != cudaSuccess)
+        return LTPG_ERR_CUDA;
     uint32_t err = 0;  // copied behind the kernels: one wait for both
     if (cudaMemcpyAsync(&err, &d->ctl->error, sizeof err, cudaMemcpyDeviceToHost, s) != cudaSuccess) return LTPG_ERR_CUDA;
     if (cudaStreamSynchronize(s) != cudaSuccess) return LTPG_ERR_CUDA;
