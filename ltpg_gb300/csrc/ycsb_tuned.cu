@@ -50,7 +50,8 @@ struct YcsbTunedArgs {
     uint32_t *bucket_counts;
     uint32_t ways, stage_entries;
     uint32_t filter;
-    uint32_t lpt;  // lanes per transaction of the one-op-per-lane kernels: stride (at most 32) rounded up to a power of two
+    uint32_t grp;  // transactions of a warp's step in the cooperative execute kernel: 32 / k
+    uint32_t lpt;  // lanes per transaction of the late reads: stride (at most 32) rounded up to a power of two
     uint32_t late; // late reads: 0 off, 1 in the check kernel's tiles, 2 in a kernel of their own,
                    // 3 write-first registration
     uint32_t *wbits;  // write-first: one bit per key, set for keys an update of the batch writes
@@ -884,15 +885,35 @@ __global__ void __launch_bounds__(BS) ycsb_exec_fast(YcsbTunedArgs a, uint32_t l
 }
 
 // ---- cooperative execute+register: one op per lane, rows read by 5 lanes ----
-// A warp takes whole transactions, lpt lanes each (the stride rounded up to a
-// power of two <= 32; lanes past the stride hold padding ops).  Each lane
-// registers its own op; then the rows of the
+// A warp takes whole transactions (warp_lanes).  Each lane registers its own op; then the rows of the
 // warp's reads are fetched six at a time, five lanes per row, each lane one
 // contiguous 16-byte chunk, so a row costs one or two cache-line requests
 // instead of five.  The five chunks are xor-folded within their lane group and
 // handed back to the lane that owns the op.
 // kReads = false (late reads): registration only; the rows are read after the
 // check, by the committed transactions alone (late_read_tile).
+// A warp's step takes grp = 32 / k consecutive transactions, k lanes each (10
+// operations: three transactions on 30 lanes, where lanes rounded up to a power
+// of two held two; 65,536 x 10: 19.7 -> 17.1 us.  The late reads keep the power
+// of two: this layout cost them 16 % at 16 operations).  Step s of the batch's
+// grp-transaction steps; this lane's transaction is s * grp + g, its op j; lanes
+// past the last transaction (g >= grp) hold none.
+struct WarpLanes {
+    uint32_t g, j;
+};
+__device__ __forceinline__ WarpLanes warp_lanes(const YcsbTunedArgs &a) {
+    const uint32_t lane = threadIdx.x & 31u;
+    return WarpLanes{lane / a.k, lane % a.k};
+}
+// Sum over a transaction's lanes, valid in its lane j = 0.
+__device__ __forceinline__ unsigned long long txn_sum(unsigned long long part, uint32_t j, uint32_t k) {
+    for (uint32_t o = 1; o < k; o <<= 1) {
+        const unsigned long long x = __shfl_down_sync(FULL, part, o);
+        if (j + o < k) part += x;
+    }
+    return part;
+}
+
 // kDedupe: one registration per distinct (key, kind), of a warp by match_any
 // (DEDUPE_WARP) or of the block (DEDUPE_BLOCK), by the first thread with it,
 // which holds the smallest TID.  For a block: a bucket of a table in shared
@@ -927,26 +948,24 @@ __device__ __forceinline__ void coop_exec_loop(const YcsbTunedArgs &a, StageEnt 
     uint32_t steps = 0;  // left before the table is cleared
     if (kTable) ops_tab = op_table<BS>();
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t lpt = a.lpt;  // lanes per transaction, a power of two
-    const uint32_t lsh = (uint32_t)__ffs(lpt) - 1u;
     const uint32_t groups = a.ways ? a.stage_entries / a.ways : 0u;
-    const uint64_t nw = (uint64_t)a.B << lsh;
-    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
-    // lanes that register before their row reads: all where no filter is asked
-    // for and the batch takes more than two steps
-    const uint64_t early = kFilter || nw <= 2u * step ? step / 8u : ~0ull;
+    const WarpLanes l = warp_lanes(a);
+    const uint32_t j = l.j, wpb = blockDim.x >> 5, warp = threadIdx.x >> 5;
+    const uint32_t n_steps = (a.B + a.grp - 1u) / a.grp, step = gridDim.x * wpb;  // warps' steps
+    // steps that register before their row reads: all where no filter is asked
+    // for and a warp takes more than two
+    const uint32_t early = kFilter || n_steps <= 2u * step ? step / 8u : ~0u;
     bool scans = false;  // some read of this thread's was a range scan
-    const uint32_t j = threadIdx.x & (lpt - 1u);  // blocks start at whole transactions
-    auto op_at = [&](uint64_t v) {
-        return v < nw && j < a.stride ? __ldg(a.ops + (v >> lsh) * a.stride + j) : LTPG_YCSB_OP_PAD;
+    auto txn_at = [&](uint32_t s) { return s < n_steps && l.g < a.grp ? s * a.grp + l.g : ~0u; };
+    auto op_at = [&](uint32_t t) {
+        return t < a.B ? __ldg(a.ops + (uint64_t)t * a.stride + j) : LTPG_YCSB_OP_PAD;
     };
-    uint32_t next = op_at((uint64_t)blockIdx.x * blockDim.x + threadIdx.x);  // one step ahead of its use
-    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < nw; base += step) {
-        const uint64_t v = base + threadIdx.x;
-        const bool act = v < nw;
-        const uint32_t t = (uint32_t)(v >> lsh);
+    uint32_t next = op_at(txn_at(blockIdx.x * wpb + warp));  // one step ahead of its use
+    for (uint32_t base = blockIdx.x * wpb; base < n_steps; base += step) {
+        const uint32_t t = txn_at(base + warp);
+        const bool act = t < a.B;
         const uint32_t w = next;
-        next = op_at(v + step);
+        next = op_at(txn_at(base + step + warp));
         bool valid = act && !ycsb_is_pad(w);
         const uint32_t key = ycsb_key(w);
         if (valid && key >= a.n) {
@@ -1029,7 +1048,7 @@ __device__ __forceinline__ void coop_exec_loop(const YcsbTunedArgs &a, StageEnt 
             *reinterpret_cast<volatile uint32_t *>(&e->dig_ok) = 1u;
         }
         unsigned long long part = rd ? x * (2ull * j + 1ull) : 0ull;
-        for (uint32_t o = lpt >> 1; o >= 1; o >>= 1) part += __shfl_xor_sync(FULL, part, o);
+        part = txn_sum(part, j, a.k);
         if (act && j == 0u) a.results[t] = (int64_t)part;
     }
     // Range scans: the keys after each scan's first, in a second pass over the
@@ -1038,12 +1057,10 @@ __device__ __forceinline__ void coop_exec_loop(const YcsbTunedArgs &a, StageEnt 
     // batches).  The same thread leads a transaction in both passes, so its
     // result is completed in program order.
     if (__syncthreads_or(scans)) {
-        for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < nw; base += step) {
-            const uint64_t v = base + threadIdx.x;
-            const bool act = v < nw;
-            const uint32_t t = (uint32_t)(v >> lsh);
-            const uint32_t j = (uint32_t)v & (lpt - 1u);
-            const uint32_t w = act && j < a.stride ? __ldg(a.ops + (uint64_t)t * a.stride + j) : LTPG_YCSB_OP_PAD;
+        for (uint32_t base = blockIdx.x * wpb; base < n_steps; base += step) {
+            const uint32_t t = txn_at(base + warp);
+            const bool act = t < a.B;
+            const uint32_t w = op_at(t);
             const bool rd = act && !ycsb_is_pad(w) && ycsb_key(w) < a.n && ycsb_span(w) != 0u;
             const uint32_t key = ycsb_key(w);
             const uint32_t last = rd ? (uint32_t)scan_last(w, a.n) : 0u;
@@ -1082,7 +1099,7 @@ __device__ __forceinline__ void coop_exec_loop(const YcsbTunedArgs &a, StageEnt 
             // the first pass added x_first * (2j + 1); the read's term is
             // x_all * (2j + 1): add the difference (mod 2^64)
             unsigned long long part = rd ? (xa - xf) * (2ull * j + 1ull) : 0ull;
-            for (uint32_t o = lpt >> 1; o >= 1; o >>= 1) part += __shfl_xor_sync(FULL, part, o);
+            part = txn_sum(part, j, a.k);
             if (act && j == 0u && part) a.results[t] = (int64_t)((unsigned long long)a.results[t] + part);
         }
     }
@@ -1353,6 +1370,9 @@ static void (*coop_kernel(int sel))(YcsbTunedArgs) {
     }
 }
 
+// Lanes of the cooperative execute kernel over the whole batch.
+static uint64_t lanes_of(const YcsbTunedArgs &a) { return 32ull * ((a.B + a.grp - 1u) / a.grp); }
+
 // A batch of up to about eight waves of lanes.  In one, a block registers a key
 // once whatever is asked for (65,536 x 10: theta 0.99 29 -> 21 us, 0 and 0.6
 // within 1 us); beyond, the barrier per step costs more than it saves (2^18 x 10
@@ -1360,14 +1380,14 @@ static void (*coop_kernel(int sel))(YcsbTunedArgs) {
 // kernel (65,536 x 10: 29.5 -> 27 us a batch); beyond, its early blocks are in
 // the way (2^20 x 10: 240 -> 242 us; with staging 414 -> 427).
 static bool few_waves(const ltpg_ctx *c, const YcsbTunedArgs &a) {
-    return (uint64_t)a.B * a.lpt <= 8192ull * c->sm_count;
+    return lanes_of(a) <= 8192ull * c->sm_count;
 }
 
 // reads = false: registration only (late reads)
 static void launch_coop(ltpg_ctx *c, const YcsbTunedArgs &a, bool stage, bool reads) {
     const LaunchCfg &L = c->launch_y;
     const size_t smem = stage ? 2 * STAGE_WORDS * sizeof(uint32_t) + (size_t)a.stage_entries * sizeof(StageEnt) : 0;
-    const uint64_t nw = (uint64_t)a.B * a.lpt;
+    const uint64_t nw = lanes_of(a);
     const int sel = !stage && few_waves(c, a) ? (L.filter ? 9 : 8) : (stage ? 4 : 0) | (L.filter ? 2 : 0) | (L.dedupe ? 1 : 0);
     void (*k)(YcsbTunedArgs) = with_block(L.block, [&](auto bs) {
         constexpr int BS = decltype(bs)::value;
@@ -1476,6 +1496,7 @@ cudaError_t ycsb_run_tuned(ltpg_ctx *c, Slot &s, int mode) {
     a.B = s.n_txn;
     a.k = s.k;
     a.stride = s.stride;
+    a.grp = 32u / s.k;
     a.lpt = 4;
     while (a.lpt < s.stride) a.lpt <<= 1;
     a.tile = tuned_tile(s.stride, threads, per_thread);  // at most; small batches take less, below
@@ -1537,7 +1558,7 @@ cudaError_t ycsb_run_tuned(ltpg_ctx *c, Slot &s, int mode) {
     const uint32_t n_tiles = (a.B + a.tile - 1) / a.tile;
     if (persistent) {
         // a lane per op in the first phase
-        const uint64_t blocks = std::max<uint64_t>(n_tiles, ((uint64_t)a.B * a.lpt + threads - 1) / threads);
+        const uint64_t blocks = std::max<uint64_t>(n_tiles, (lanes_of(a) + threads - 1) / threads);
         const uint32_t grid = (uint32_t)std::min<uint64_t>(resident, blocks);
         prof_mark(c, 0);
         void *args[] = {&a};
