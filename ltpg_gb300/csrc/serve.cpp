@@ -70,7 +70,7 @@ struct DevSlot {
     bool busy = false;
     cudaEvent_t start = nullptr, done_c = nullptr, done_y = nullptr;
     Pinned c_flags, c_res, y_flags, y_res;  // results, copied back behind the kernels
-    Pinned ctl;                             // and both engines' control blocks as the batch leaves them
+    DevCtl *ctl = nullptr;                  // both engines' control blocks as the batch leaves them (behind c_res)
     uint64_t first_id = 0;
     uint32_t n = 0, n_c = 0, n_y = 0;
     std::vector<uint32_t> map;      // per request: (index in its part << 1) | (1 for YCSB)
@@ -168,8 +168,7 @@ bool complete_oldest(ltpg_server *s, bool block) {
     cudaEventElapsedTime(&ms_c, d.start, d.done_c);
     cudaEventElapsedTime(&ms_y, d.start, d.done_y);
     s->dev_sum += std::max(ms_c, ms_y) * 1e-3;
-    const DevCtl *ctl = d.ctl.as<DevCtl>();
-    s->look |= (d.n_c && ctl[0].error) || (d.n_y && ctl[1].error);
+    s->look |= (d.n_c && d.ctl[0].error) || (d.n_y && d.ctl[1].error);
     const uint8_t *cf = d.c_flags.as<uint8_t>(), *yf = d.y_flags.as<uint8_t>();
     const int64_t *cr = d.c_res.as<int64_t>(), *yr = d.y_res.as<int64_t>();
     for (uint32_t i = 0; i < d.n; ++i) {
@@ -239,7 +238,7 @@ int close_batch(ltpg_server *s, bool block) {
         const Slot &es = s->tc->slots[slot];
         cudaMemcpyAsync(d.c_flags.p, es.flags, s->form_c, cudaMemcpyDeviceToHost, s->cs_c);
         cudaMemcpyAsync(d.c_res.p, es.results, (size_t)s->form_c * 8, cudaMemcpyDeviceToHost, s->cs_c);
-        cudaMemcpyAsync(d.ctl.p, s->tc->ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, s->cs_c);
+        cudaMemcpyAsync(d.ctl, s->tc->ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, s->cs_c);
     } else {
         cudaEventRecord(g.up_c, s->cp_c);
         cudaStreamWaitEvent(s->cs_c, d.start, 0);
@@ -258,7 +257,7 @@ int close_batch(ltpg_server *s, bool block) {
         const Slot &es = s->yc->slots[slot];
         cudaMemcpyAsync(d.y_flags.p, es.flags, s->form_y, cudaMemcpyDeviceToHost, s->cs_y);
         cudaMemcpyAsync(d.y_res.p, es.results, (size_t)s->form_y * 8, cudaMemcpyDeviceToHost, s->cs_y);
-        cudaMemcpyAsync(d.ctl.as<DevCtl>() + 1, s->yc->ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, s->cs_y);
+        cudaMemcpyAsync(d.ctl + 1, s->yc->ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, s->cs_y);
     } else {
         cudaEventRecord(g.up_y, s->cp_y);
         cudaStreamWaitEvent(s->cs_y, d.start, 0);
@@ -471,8 +470,9 @@ int ltpg_server_open(ltpg_ctx *tc, ltpg_ctx *yc, const ltpg_server_cfg *cfg, ltp
              cudaEventCreateWithFlags(&g.up_y, cudaEventDisableTiming) == cudaSuccess;
     }
     for (auto &d : s->dev) {
-        ok = ok && d.c_flags.reserve(m) && d.c_res.reserve(m * 8) && d.y_flags.reserve(m) && d.y_res.reserve(m * 8) &&
-             d.ctl.reserve(2 * sizeof(DevCtl));
+        ok = ok && d.c_flags.reserve(m) && d.c_res.reserve(m * 8 + 2 * sizeof(DevCtl)) && d.y_flags.reserve(m) &&
+             d.y_res.reserve(m * 8);
+        if (ok) d.ctl = reinterpret_cast<DevCtl *>(d.c_res.as<int64_t>() + m);
         ok = ok && cudaEventCreate(&d.start) == cudaSuccess && cudaEventCreate(&d.done_c) == cudaSuccess &&
              cudaEventCreate(&d.done_y) == cudaSuccess;
     }
