@@ -173,6 +173,9 @@ typedef struct {
     uint32_t line_off;
 } ltpg_tpcc_txn;
 
+/* A line whose item (>= 100,000) or supply warehouse (>= W) is out of range is
+ * reported as LTPG_ERR_BOUNDS, like a record out of range; its NewOrder does
+ * not commit and writes nothing. */
 typedef struct {
     uint32_t i_id;
     uint16_t supply_w;

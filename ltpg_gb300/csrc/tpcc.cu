@@ -341,6 +341,11 @@ __device__ __forceinline__ bool result_read(const TpccDev &db, const ltpg_tpcc_t
     }
 }
 
+// In a tile's conflict flags, above the flag byte: some order line's supply
+// warehouse is another one; some order line is out of range (its NewOrder does
+// not commit: the write-back takes a committed order's lines as they are).
+constexpr uint32_t FL_REMOTE = 0x100u, FL_BAD_LINE = 0x200u;
+
 // ---- plain phase 1: execute + register (KERNEL_EXECUTE, TF/tp.cu:24-54) ----
 __global__ void __launch_bounds__(PBS) tpcc_exec_plain(const ltpg_tpcc_txn *__restrict__ txns, uint32_t B,
                                                        const ltpg_tpcc_line *__restrict__ lines,
@@ -418,7 +423,10 @@ __global__ void __launch_bounds__(PBS) tpcc_check_plain(const ltpg_tpcc_txn *__r
         ltpg_tpcc_line ln{0, 0, 0};
         if (tpcc_kind(x.kind_info) == LTPG_TPCC_NEWORDER && j >= 5) {
             ln = load_line(lines, (uint64_t)x.line_off + (j - 5) / 3);
-            if (!line_valid(ln, db.W)) continue;
+            if (!line_valid(ln, db.W)) {
+                atomicOr(&fl[i], FL_BAD_LINE);
+                continue;
+            }
         }
         const TpccOp op = tpcc_op(x, j, ln, db.strict);
         const ulonglong2 s = ld_slot(reg + db.base[op.table] + op.row);
@@ -432,13 +440,14 @@ __global__ void __launch_bounds__(PBS) tpcc_check_plain(const ltpg_tpcc_txn *__r
     __syncthreads();
     if (threadIdx.x < nt) {
         uint32_t f = fl[threadIdx.x];
-        if (h.ok[threadIdx.x] && commits(f)) f |= LTPG_FLAG_COMMIT;
+        if (h.ok[threadIdx.x] && !(f & FL_BAD_LINE) && commits(f)) f |= LTPG_FLAG_COMMIT;
         if (txn_not_found(h.x[threadIdx.x])) f |= LTPG_FLAG_NOT_FOUND;
         flags[t0 + threadIdx.x] = (uint8_t)f;
     }
 }
 
-// Write op q of a committed transaction.  NewOrder: 0 ORDER insert, 1
+// Write op q of a committed transaction (its order lines are in range: one that
+// is not keeps its NewOrder from committing).  NewOrder: 0 ORDER insert, 1
 // NEW-ORDER insert, 2+2i stock update of line i, 3+2i ORDER-LINE insert of
 // line i.  Payment: 0 W_YTD add, 1 D_YTD add, 2 customer update, 3 HISTORY
 // insert.  Delivery: 0 NEW-ORDER delete, 1 ORDER carrier, 2 ORDER-LINE delivery
@@ -1078,7 +1087,7 @@ __device__ __forceinline__ void write_head(const TpccDev &db, const ltpg_tpcc_tx
     }
 }
 
-// Line li of a committed NewOrder: the stock update (atomic: an order may list
+// Line li of a committed NewOrder, which is in range: the stock update (atomic: an order may list
 // a row twice, see tpcc_apply_write) and the ORDER-LINE insert.
 __device__ __forceinline__ void write_line(const TpccDev &db, const ltpg_tpcc_txn &x, uint32_t li,
                                            const ltpg_tpcc_line &ln) {
@@ -1102,8 +1111,6 @@ __device__ __forceinline__ void write_line(const TpccDev &db, const ltpg_tpcc_tx
     st_cols2(o + OL_DELIVERY_D, 0u, ln.qty);
     st_cols2(o + OL_AMOUNT, (uint64_t)ln.qty * price, info);
 }
-
-constexpr uint32_t FL_REMOTE = 0x100u;  // in a tile's flags: some line's supply warehouse is another one
 
 // hot: 11 W 64-bit sums in shared memory (W <= HOT_SMEM_MAX_W), or null.
 template <uint32_t P, uint32_t T, bool kClaim>
@@ -1165,6 +1172,8 @@ __device__ __forceinline__ TxnCounts tpcc_checkwb_tiles(const TpccTunedArgs &a, 
                 if (!kClaim || (any_multi && ((ml[q] >> li) & 1u)))
                     g |= conflicts_of(ld_slot(a.reg + a.db.base[LTPG_T_ORDERLINE] + tpcc_ol_row(y.w, y.c, li)),
                                       OPF_WRITE, t0 + q, epoch);
+            } else {
+                g |= FL_BAD_LINE;
             }
             if (g & ~fl[q]) atomicOr(&fl[q], g);
         }
@@ -1172,7 +1181,7 @@ __device__ __forceinline__ TxnCounts tpcc_checkwb_tiles(const TpccTunedArgs &a, 
         if (i < P) {  // whole warps
             const uint32_t all = fl[i];
             f = all & (LTPG_FLAG_RAW | LTPG_FLAG_WAR | LTPG_FLAG_WAW);
-            com = ok && commits(f);
+            com = ok && !(all & FL_BAD_LINE) && commits(f);
             if (com) f |= LTPG_FLAG_COMMIT;
             if (i < nt) {
                 if (txn_not_found(x)) f |= LTPG_FLAG_NOT_FOUND;
