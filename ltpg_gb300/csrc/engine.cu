@@ -400,8 +400,7 @@ int slot_prepare_ycsb(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint32_t k, ui
     return LTPG_OK;
 }
 
-int slot_prepare_tpcc(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint64_t n_lines, uint64_t txn_base,
-                      bool reads_orders, Slot **out) {
+int slot_prepare_tpcc(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint64_t n_lines, uint64_t txn_base, Slot **out) {
     Slot *s = get_slot(c, slot);
     if (!s) return fail(c, LTPG_ERR_INVALID, "bad slot or batch");
     if (!c->tpcc.W) return fail(c, LTPG_ERR_STATE, "no TPC-C tables loaded");
@@ -416,14 +415,18 @@ int slot_prepare_tpcc(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint64_t n_lin
     }
     int r = ensure_outputs(c, *s, n_txn);
     if (r) return r;
-    if (s->workload != LTPG_WORKLOAD_TPCC || s->n_txn != n_txn || s->reads_orders != reads_orders) drop_graphs(c);
+    if (s->workload != LTPG_WORKLOAD_TPCC || s->n_txn != n_txn) drop_graphs(c);
     s->workload = LTPG_WORKLOAD_TPCC;
-    s->reads_orders = reads_orders;
     s->n_txn = n_txn;
     s->n_lines = (uint32_t)n_lines;
     s->txn_base = txn_base;
     *out = s;
     return LTPG_OK;
+}
+
+void slot_set_reads_orders(ltpg_ctx *c, Slot &s, bool reads_orders) {
+    if (s.reads_orders != reads_orders) drop_graphs(c);
+    s.reads_orders = reads_orders;
 }
 
 int ctx_fail(ltpg_ctx *c, int code, const char *msg) { return fail(c, code, msg); }
@@ -462,14 +465,15 @@ int upload_tpcc(ltpg_ctx *c, uint32_t slot, const ltpg_tpcc_batch *b, cudaStream
     if (!c || !b) return c ? fail(c, LTPG_ERR_INVALID, "bad slot or batch") : LTPG_ERR_INVALID;
     if (!b->txns || (b->n_lines && !b->lines && !packed)) return fail(c, LTPG_ERR_INVALID, "null batch array");
     Slot *s = nullptr;
+    int r = slot_prepare_tpcc(c, slot, b->n_txn, b->n_lines, b->txn_base, &s);
+    if (r) return r;
     // 64 records spread over the batch tell a mix with OrderStatus or Delivery
     bool reads_orders = false;
     for (uint32_t i = 0; i < 64u && b->n_txn >= CLAIM_MIN_TXNS; ++i) {
         const uint32_t kind = tpcc_kind(b->txns[(uint64_t)b->n_txn * i / 64u].kind_info);
         reads_orders |= kind == LTPG_TPCC_ORDERSTATUS || kind == LTPG_TPCC_DELIVERY;
     }
-    int r = slot_prepare_tpcc(c, slot, b->n_txn, b->n_lines, b->txn_base, reads_orders, &s);
-    if (r) return r;
+    slot_set_reads_orders(c, *s, reads_orders);
     CK(cudaMemcpyAsync(s->txns, b->txns, (uint64_t)b->n_txn * sizeof(ltpg_tpcc_txn), cudaMemcpyHostToDevice, st),
        "upload txns");
     if (b->n_lines && packed) {

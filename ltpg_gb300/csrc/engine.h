@@ -205,8 +205,9 @@ void drop_graphs_ctx(ltpg_ctx *c);
 // invalidation) and records the shape; the caller fills the batch buffers.
 int slot_prepare_ycsb(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint32_t k, uint32_t n_updates, Slot **out);
 constexpr uint32_t CLAIM_MIN_TXNS = 131072;  // tpcc.cu, tpcc_claims
-int slot_prepare_tpcc(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint64_t n_lines, uint64_t txn_base,
-                      bool reads_orders, Slot **out);
+int slot_prepare_tpcc(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint64_t n_lines, uint64_t txn_base, Slot **out);
+// Sets a prepared TPC-C slot's reads_orders.
+void slot_set_reads_orders(ltpg_ctx *c, Slot &s, bool reads_orders);
 // Makes generator g's batch batch_id in slot `slot` on stream st (gen_dev.cu).
 int gen_device_batch(ltpg_ctx *c, ltpg_gen *g, uint64_t batch_id, uint32_t slot, cudaStream_t st);
 // Makes room for `batches` more batch epochs before a launch (resets the

@@ -934,9 +934,9 @@ int gen_tpcc(ltpg_ctx *c, ltpg_gen *g, uint64_t batch_id, uint32_t slot, cudaStr
     if (max_lines > c->cfg.max_lines)
         return ctx_fail(c, LTPG_ERR_INVALID, "device generation needs max_lines >= 15 n_txn");
     Slot *s = nullptr;
-    int r = slot_prepare_tpcc(c, slot, p.n_txn, max_lines, g->txn_base,
-                              p.n_txn >= CLAIM_MIN_TXNS && (p.orderstatus_pct || p.delivery_pct), &s);
+    int r = slot_prepare_tpcc(c, slot, p.n_txn, max_lines, g->txn_base, &s);
     if (r) return r;
+    slot_set_reads_orders(c, *s, p.n_txn >= CLAIM_MIN_TXNS && (p.orderstatus_pct || p.delivery_pct));
     cudaError_t e = cudaSuccess;
     if (!g->dev && (e = bind_tpcc(g, c->device)) != cudaSuccess) return ctx_cuda_fail(c, e, "generator state to device");
     ltpg_gen_dev *d = g->dev;
