@@ -281,6 +281,7 @@ int ltpg_db_load_tpcc(ltpg_ctx *c, uint64_t seed, uint32_t W) {
     dev_free(c->tpcc.claim);
     dev_free(c->tpcc.stock_w);
     c->tpcc = TpccDb{};
+    for (auto &s : c->slots) s.reads_orders = false;
     uint64_t total = 0;
     for (uint32_t t = 0; t < LTPG_TPCC_TABLES; ++t) {
         c->tpcc.rows[t] = tpcc_rows(t, W);
@@ -415,7 +416,10 @@ int slot_prepare_tpcc(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint64_t n_lin
     }
     int r = ensure_outputs(c, *s, n_txn);
     if (r) return r;
-    if (s->workload != LTPG_WORKLOAD_TPCC || s->n_txn != n_txn) drop_graphs(c);
+    if (s->workload != LTPG_WORKLOAD_TPCC || s->n_txn != n_txn) {
+        drop_graphs(c);
+        s->reads_orders = false;
+    }
     s->workload = LTPG_WORKLOAD_TPCC;
     s->n_txn = n_txn;
     s->n_lines = (uint32_t)n_lines;
@@ -424,9 +428,10 @@ int slot_prepare_tpcc(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint64_t n_lin
     return LTPG_OK;
 }
 
-void slot_set_reads_orders(ltpg_ctx *c, Slot &s, bool reads_orders) {
-    if (s.reads_orders != reads_orders) drop_graphs(c);
-    s.reads_orders = reads_orders;
+void slot_saw_order_reads(ltpg_ctx *c, Slot &s) {
+    const bool claims = tpcc_claims(s, c->tpcc.W);
+    s.reads_orders = true;
+    if (claims != tpcc_claims(s, c->tpcc.W)) drop_graphs(c);
 }
 
 int ctx_fail(ltpg_ctx *c, int code, const char *msg) { return fail(c, code, msg); }
@@ -468,12 +473,13 @@ int upload_tpcc(ltpg_ctx *c, uint32_t slot, const ltpg_tpcc_batch *b, cudaStream
     int r = slot_prepare_tpcc(c, slot, b->n_txn, b->n_lines, b->txn_base, &s);
     if (r) return r;
     // 64 records spread over the batch tell a mix with OrderStatus or Delivery
-    bool reads_orders = false;
     for (uint32_t i = 0; i < 64u && b->n_txn >= CLAIM_MIN_TXNS; ++i) {
         const uint32_t kind = tpcc_kind(b->txns[(uint64_t)b->n_txn * i / 64u].kind_info);
-        reads_orders |= kind == LTPG_TPCC_ORDERSTATUS || kind == LTPG_TPCC_DELIVERY;
+        if (kind == LTPG_TPCC_ORDERSTATUS || kind == LTPG_TPCC_DELIVERY) {
+            slot_saw_order_reads(c, *s);
+            break;
+        }
     }
-    slot_set_reads_orders(c, *s, reads_orders);
     CK(cudaMemcpyAsync(s->txns, b->txns, (uint64_t)b->n_txn * sizeof(ltpg_tpcc_txn), cudaMemcpyHostToDevice, st),
        "upload txns");
     if (b->n_lines && packed) {

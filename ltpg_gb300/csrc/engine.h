@@ -105,9 +105,12 @@ struct Slot {
     // TPC-C
     uint32_t n_lines = 0;
     uint64_t txn_base = 0;
-    // A batch of CLAIM_MIN_TXNS or more has OrderStatus or Delivery transactions
-    // (a device-made batch's mix; a sample of an uploaded one's): says which
-    // registration is likely faster, both give the same outcome.
+    // A batch of this size in this slot has had OrderStatus or Delivery
+    // transactions (a device-made batch's mix; a sample of an uploaded one's,
+    // which misses rare ones in some batches: so it stays set until the size
+    // changes, or batches of one mix would change kernels and captured graphs
+    // back and forth).  Says which registration is likely faster; both give the
+    // same outcome.
     bool reads_orders = false;
     ltpg_tpcc_txn *txns = nullptr;
     ltpg_tpcc_line *lines = nullptr;
@@ -206,8 +209,10 @@ void drop_graphs_ctx(ltpg_ctx *c);
 int slot_prepare_ycsb(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint32_t k, uint32_t n_updates, Slot **out);
 constexpr uint32_t CLAIM_MIN_TXNS = 131072;  // tpcc.cu, tpcc_claims
 int slot_prepare_tpcc(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint64_t n_lines, uint64_t txn_base, Slot **out);
-// Sets a prepared TPC-C slot's reads_orders.
-void slot_set_reads_orders(ltpg_ctx *c, Slot &s, bool reads_orders);
+// Sets a prepared TPC-C slot's reads_orders; captured graphs go if its kernels change.
+void slot_saw_order_reads(ltpg_ctx *c, Slot &s);
+// Whether the slot's batch claims its inserted rows (tpcc.cu).
+bool tpcc_claims(const Slot &s, uint32_t W);
 // Makes generator g's batch batch_id in slot `slot` on stream st (gen_dev.cu).
 int gen_device_batch(ltpg_ctx *c, ltpg_gen *g, uint64_t batch_id, uint32_t slot, cudaStream_t st);
 // Makes room for `batches` more batch epochs before a launch (resets the

@@ -1346,7 +1346,7 @@ static cudaError_t tpcc_launch_block(ltpg_ctx *c, const TpccTunedArgs &a, int mo
 // 78; W = 8, 2^19: 114 -> 116).  They do not where orders are read or delivered
 // in the batch that makes them (the five-transaction mix at 2^18: 110 -> 118) or
 // the ids of a warehouse wrap in it (W = 4, 2^20: 161 -> 244).
-static bool tpcc_claims(const Slot &s, uint32_t W) {
+bool tpcc_claims(const Slot &s, uint32_t W) {
     return !s.reads_orders && W >= 16u && s.n_txn >= CLAIM_MIN_TXNS && s.n_txn <= 32768ull * W;
 }
 
