@@ -281,7 +281,6 @@ int ltpg_db_load_tpcc(ltpg_ctx *c, uint64_t seed, uint32_t W) {
     dev_free(c->tpcc.claim);
     dev_free(c->tpcc.stock_w);
     c->tpcc = TpccDb{};
-    for (auto &s : c->slots) s.reads_orders = false;
     uint64_t total = 0;
     for (uint32_t t = 0; t < LTPG_TPCC_TABLES; ++t) {
         c->tpcc.rows[t] = tpcc_rows(t, W);
@@ -293,13 +292,13 @@ int ltpg_db_load_tpcc(ltpg_ctx *c, uint64_t seed, uint32_t W) {
     CK(dev_alloc(&c->tpcc.reg, total), "alloc TPC-C registration table");
     CK(dev_alloc(&c->tpcc.name_idx, c->tpcc.rows[LTPG_T_CUSTOMER]), "alloc customer name index");
     CK(dev_alloc(&c->tpcc.name_dir, 10ull * W * NAME_DIR_LEN), "alloc customer name directory");
-    CK(dev_alloc(&c->tpcc.claim, claim_total_words(W)), "alloc claim bitmaps");
-    CK(dev_alloc(&c->tpcc.stock_w, c->tpcc.rows[LTPG_T_STOCK]), "alloc stock writers");
     c->tpcc.n_slots = total;
     c->tpcc.W = W;
     c->tpcc_seed = seed;
     CK(tpcc_init_tables(c), "init TPC-C tables");
     CK(tpcc_build_name_index(c), "build customer name index");
+    for (auto &s : c->slots)  // the batches that the slots hold may run on the new tables
+        if (s.workload == LTPG_WORKLOAD_TPCC) slot_pick_registration(c, s, false);
     return ltpg_sync(c);
 }
 
@@ -428,10 +427,23 @@ int slot_prepare_tpcc(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint64_t n_lin
     return LTPG_OK;
 }
 
-void slot_saw_order_reads(ltpg_ctx *c, Slot &s) {
-    const bool claims = tpcc_claims(s, c->tpcc.W);
-    s.reads_orders = true;
-    if (claims != tpcc_claims(s, c->tpcc.W)) drop_graphs(c);
+void slot_pick_registration(ltpg_ctx *c, Slot &s, bool order_reads) {
+    TpccDb &db = c->tpcc;
+    const bool claimed = tpcc_claims(s, db);
+    s.reads_orders |= order_reads;
+    if (claimed != tpcc_claims(s, db)) drop_graphs(c);
+    if (!tpcc_claims(s, db) || db.claim) return;
+    // on the stream that the slot's batch runs on, or that it waits for
+    cudaError_t e = dev_alloc(&db.claim, claim_total_words(db.W));
+    if (e == cudaSuccess) e = dev_alloc(&db.stock_w, db.rows[LTPG_T_STOCK]);
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(db.stock_w, 0xFF, db.rows[LTPG_T_STOCK] * sizeof(unsigned long long), c->stream);
+    if (e != cudaSuccess) {  // no room: the slots serve
+        cudaGetLastError();
+        dev_free(db.claim);
+        dev_free(db.stock_w);
+        db.no_claims = true;
+    }
 }
 
 int ctx_fail(ltpg_ctx *c, int code, const char *msg) { return fail(c, code, msg); }
@@ -473,13 +485,12 @@ int upload_tpcc(ltpg_ctx *c, uint32_t slot, const ltpg_tpcc_batch *b, cudaStream
     int r = slot_prepare_tpcc(c, slot, b->n_txn, b->n_lines, b->txn_base, &s);
     if (r) return r;
     // 64 records spread over the batch tell a mix with OrderStatus or Delivery
+    bool order_reads = false;
     for (uint32_t i = 0; i < 64u && b->n_txn >= CLAIM_MIN_TXNS; ++i) {
         const uint32_t kind = tpcc_kind(b->txns[(uint64_t)b->n_txn * i / 64u].kind_info);
-        if (kind == LTPG_TPCC_ORDERSTATUS || kind == LTPG_TPCC_DELIVERY) {
-            slot_saw_order_reads(c, *s);
-            break;
-        }
+        order_reads |= kind == LTPG_TPCC_ORDERSTATUS || kind == LTPG_TPCC_DELIVERY;
     }
+    slot_pick_registration(c, *s, order_reads);
     CK(cudaMemcpyAsync(s->txns, b->txns, (uint64_t)b->n_txn * sizeof(ltpg_tpcc_txn), cudaMemcpyHostToDevice, st),
        "upload txns");
     if (b->n_lines && packed) {

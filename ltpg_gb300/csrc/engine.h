@@ -74,9 +74,12 @@ struct TpccDb {
     RegSlot *reg = nullptr;  // flat over all tables
     uint64_t base[LTPG_TPCC_TABLES] = {};
     // Claims of a batch (tuned path): bitmaps of claim_total_words() words, and
-    // the STOCK rows' smallest writers, epoch-tagged like a slot's.
+    // the STOCK rows' smallest writers, epoch-tagged like a slot's.  0.95 MB a
+    // warehouse, taken with the first batch that claims; tables that leave no
+    // room for them do without (no_claims).
     uint32_t *claim = nullptr;
     unsigned long long *stock_w = nullptr;
+    bool no_claims = false;
     // Customer last-name index: per district its 3,000 keys
     // (min(C_LAST, 2^32 - 1) << 32 | C_ID) in ascending order.
     uint64_t *name_idx = nullptr;
@@ -209,10 +212,11 @@ void drop_graphs_ctx(ltpg_ctx *c);
 int slot_prepare_ycsb(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint32_t k, uint32_t n_updates, Slot **out);
 constexpr uint32_t CLAIM_MIN_TXNS = 131072;  // tpcc.cu, tpcc_claims
 int slot_prepare_tpcc(ltpg_ctx *c, uint32_t slot, uint32_t n_txn, uint64_t n_lines, uint64_t txn_base, Slot **out);
-// Sets a prepared TPC-C slot's reads_orders; captured graphs go if its kernels change.
-void slot_saw_order_reads(ltpg_ctx *c, Slot &s);
-// Whether the slot's batch claims its inserted rows (tpcc.cu).
-bool tpcc_claims(const Slot &s, uint32_t W);
+// Notes a prepared TPC-C slot's order reads (captured graphs go if its kernels
+// change) and makes room for its claims if it takes them.
+void slot_pick_registration(ltpg_ctx *c, Slot &s, bool order_reads);
+// Whether the slot's batch should claim its inserted rows (tpcc.cu).
+bool tpcc_claims(const Slot &s, const TpccDb &db);
 // Makes generator g's batch batch_id in slot `slot` on stream st (gen_dev.cu).
 int gen_device_batch(ltpg_ctx *c, ltpg_gen *g, uint64_t batch_id, uint32_t slot, cudaStream_t st);
 // Makes room for `batches` more batch epochs before a launch (resets the

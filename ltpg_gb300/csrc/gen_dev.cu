@@ -936,7 +936,7 @@ int gen_tpcc(ltpg_ctx *c, ltpg_gen *g, uint64_t batch_id, uint32_t slot, cudaStr
     Slot *s = nullptr;
     int r = slot_prepare_tpcc(c, slot, p.n_txn, max_lines, g->txn_base, &s);
     if (r) return r;
-    if (p.orderstatus_pct || p.delivery_pct) slot_saw_order_reads(c, *s);
+    slot_pick_registration(c, *s, p.orderstatus_pct || p.delivery_pct);
     cudaError_t e = cudaSuccess;
     if (!g->dev && (e = bind_tpcc(g, c->device)) != cudaSuccess) return ctx_cuda_fail(c, e, "generator state to device");
     ltpg_gen_dev *d = g->dev;

@@ -98,7 +98,7 @@ cudaError_t tpcc_init_tables(ltpg_ctx *c) {
 
 cudaError_t tpcc_clear_slots(ltpg_ctx *c) {
     const cudaError_t e = cudaMemsetAsync(c->tpcc.reg, 0xFF, c->tpcc.n_slots * sizeof(RegSlot), c->stream);
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess || !c->tpcc.stock_w) return e;
     return cudaMemsetAsync(c->tpcc.stock_w, 0xFF, c->tpcc.rows[LTPG_T_STOCK] * sizeof(unsigned long long), c->stream);
 }
 
@@ -1346,8 +1346,8 @@ static cudaError_t tpcc_launch_block(ltpg_ctx *c, const TpccTunedArgs &a, int mo
 // 78; W = 8, 2^19: 114 -> 116).  They do not where orders are read or delivered
 // in the batch that makes them (the five-transaction mix at 2^18: 110 -> 118) or
 // the ids of a warehouse wrap in it (W = 4, 2^20: 161 -> 244).
-bool tpcc_claims(const Slot &s, uint32_t W) {
-    return !s.reads_orders && W >= 16u && s.n_txn >= CLAIM_MIN_TXNS && s.n_txn <= 32768ull * W;
+bool tpcc_claims(const Slot &s, const TpccDb &db) {
+    return !db.no_claims && !s.reads_orders && db.W >= 16u && s.n_txn >= CLAIM_MIN_TXNS && s.n_txn <= 32768ull * db.W;
 }
 
 cudaError_t tpcc_run_tuned(ltpg_ctx *c, Slot &s, int mode) {
@@ -1372,7 +1372,7 @@ cudaError_t tpcc_run_tuned(ltpg_ctx *c, Slot &s, int mode) {
     a.any = a.multi + a.claim_words;
     a.sl_bits = a.any + 2;
     a.stock_w = c->tpcc.stock_w;
-    const bool claim = mode != LTPG_MODE_PERSISTENT && tpcc_claims(s, a.db.W);
+    const bool claim = mode != LTPG_MODE_PERSISTENT && c->tpcc.claim && tpcc_claims(s, c->tpcc);
     switch (c->launch_c.block) {
     case 256: return tpcc_launch_block<256>(c, a, mode, claim);
     case 512: return tpcc_launch_block<512>(c, a, mode, claim);
