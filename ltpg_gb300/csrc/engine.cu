@@ -759,7 +759,11 @@ int ltpg_host_wait(ltpg_ctx *c, uint32_t slot) {
     Slot *s = get_slot(c, slot);
     if (!s) return c ? fail(c, LTPG_ERR_INVALID, "bad slot") : LTPG_ERR_INVALID;
     if (s->done) CK(cudaEventSynchronize(s->done), "wait for the slot");
-    const bool clean = s->submitted && s->left->error == 0u;
+    // a slot without a submitted batch has nothing to wait for: the error word
+    // as it is now, not behind the other slots' batches
+    DevCtl now;
+    if (!s->submitted) CK(cudaMemcpy(&now, c->ctl, sizeof now, cudaMemcpyDeviceToHost), "read control block");
+    const bool clean = (s->submitted ? s->left : &now)->error == 0u;
     s->submitted = false;
     return clean ? LTPG_OK : check_device_error(c);
 }
