@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(TB) ycsb_gen_vals(YcsbGenArgs a, const uint32_
             for (uint32_t q = 0; q < 4; ++q)
                 if (!ycsb_is_pad(w[q]) && ycsb_is_update(w[q])) a.vals[v++] = splitmix64(h ^ (4u * seg + q));
         }
-        // every lane of the transaction has read its count by the shuffle above
+        __syncwarp();  // every lane of the transaction has read its count (a shuffle orders no memory access)
         if (act && seg == 0u) a.val_off[t + 1] = end;
     }
 }
