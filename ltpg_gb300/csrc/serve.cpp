@@ -351,16 +351,17 @@ int submit(ltpg_server *s, const ltpg_request *reqs, uint32_t n, uint64_t *first
     int r = progress(s);
     if (r) return r;
     if (first_id) *first_id = s->next_id;
-    double called = s->now();  // and again after every wait below
+    double now = 0;  // looked at every 32 requests and after every wait: a look takes 32 ns, packing a request 23
     for (uint32_t i = 0; i < n; ++i) {
         const ltpg_request &q = reqs[i];
+        if (!t_submit && i % 32u == 0u) now = s->now();
         if ((r = check_request(s, q))) return r;
-        const double t = t_submit ? t_submit[i] : called;
+        const double t = t_submit ? t_submit[i] : now;
         const bool lines_full =
             q.workload == LTPG_WORKLOAD_TPCC && s->form_lines + q.n > s->max_lines;
         if (s->form_n && (s->form_n >= s->max_batch || lines_full)) {
             if ((r = close_batch(s, true))) return r;
-            called = s->now();
+            now = s->now();
         }
         if (s->form_n == 0 && (r = begin_forming(s, t))) return r;
         pack(s, q, t);
