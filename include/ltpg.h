@@ -574,10 +574,14 @@ int ltpg_counters(ltpg_ctx *ctx, uint64_t *commits_total, uint64_t *kernel_launc
 /* When on, every batch run records CUDA events around each of its kernels
  * (also inside captured graphs); ltpg_kernel_times writes the durations in
  * milliseconds of the last run of a slot into ms4 = [execute, check, reads,
- * write-back].  A phase that runs inside another kernel reads 0: the tuned
+ * write-back].  A phase that runs inside another kernel reads next to nothing
+ * (two events back to back: about 2 us): the tuned
  * modes' check kernel also writes back ([execute, check+write-back, 0, 0]),
  * YCSB late reads in the check kernel give [execute, check+reads, 0,
- * write-back], and a persistent launch puts the whole batch under execute. */
+ * write-back], and a persistent launch puts the whole batch under execute.
+ * No kernel starts before the one before it has ended then; in small batches
+ * without events launches overlap, and the whole batch takes a microsecond or
+ * two less than its split says. */
 int ltpg_set_profiling(ltpg_ctx *ctx, int on);
 int ltpg_kernel_times(ltpg_ctx *ctx, uint32_t slot, float *ms4);
 

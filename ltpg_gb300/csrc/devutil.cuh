@@ -189,7 +189,8 @@ __device__ __forceinline__ void clear_stats(DevStats *st) {
 
 // A kernel whose launch may overlap the end of the one before it (launch_next):
 // its blocks come up where they find room and wait here, which hides the launch
-// (about 1 us).  What the other kernel wrote is read by plain loads only: the
+// (about 1 us; not with profiling events, whose split is of kernels one after
+// another).  What the other kernel wrote is read by plain loads only: the
 // read-only path may hold lines from before the wait.
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // In the kernel before it, whose blocks are all resident by then.

@@ -1318,7 +1318,7 @@ static cudaError_t tpcc_launch_tuned(ltpg_ctx *c, const TpccTunedArgs &a_in, int
     count_launch(c);
     // on small tiles only: the early blocks of a full wave are in the way (the
     // mix at 2^20: 283 -> 316 us; at 20,000: 21 -> 19)
-    e = launch_next(tpcc_checkwb_tuned<P, T, kClaim>, P < T, grid, threads, smem, c->stream, a);
+    e = launch_next(tpcc_checkwb_tuned<P, T, kClaim>, P < T && !c->profiling, grid, threads, smem, c->stream, a);
     if (e != cudaSuccess) return e;
     for (int m = 2; m < PROF_MARKS; ++m) prof_mark(c, m);
     return cudaSuccess;

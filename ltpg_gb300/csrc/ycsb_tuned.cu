@@ -1577,7 +1577,7 @@ cudaError_t ycsb_run_tuned(ltpg_ctx *c, Slot &s, int mode) {
     prof_mark(c, 1);
     count_launch(c);
     const uint32_t grid_cwb = std::min(n_tiles, resident);
-    e = launch_next(cwb_k, !stage && few_waves(c, a), grid_cwb, threads, smem_cwb, c->stream, a);
+    e = launch_next(cwb_k, !stage && !c->profiling && few_waves(c, a), grid_cwb, threads, smem_cwb, c->stream, a);
     if (e != cudaSuccess) return e;
     prof_mark(c, 2);
     if (late_mode == 2u) {
