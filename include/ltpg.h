@@ -405,11 +405,21 @@ typedef struct {
     uint32_t block_threads;   /* threads per block of the tuned kernels: 128, 256
                                  or 512 (TPC-C: on tiles of up to as
                                  many transactions)                             */
-    uint32_t ops_per_thread;  /* YCSB op words per thread: 1, 2, 4 or 8         */
+    uint32_t ops_per_thread;  /* YCSB op words per thread: 1, 2, 4 or 8 (2 and 4
+                                 where op_stride / ops_per_thread is a power of
+                                 two; otherwise as 1)                           */
     uint32_t blocks_per_sm;   /* cap on resident blocks per SM, 0 = occupancy   */
     uint32_t stage_ways;      /* shared-memory staging entries per hot bucket   */
-    uint32_t filter;          /* 1 = read the slot before its atomicMin         */
-    uint32_t dedupe;          /* 1 = one atomic per key per warp (match_any; TPC-C: header ops) */
+    uint32_t filter;          /* 1 = read the slot before its atomicMin (where
+                                 blocks register a key once, see dedupe, most
+                                 lanes do so with 0 too)                        */
+    uint32_t dedupe;          /* 1 = one atomic per key per warp (match_any; TPC-C:
+                                 the op on the customer or, StockLevel, the stock
+                                 row).  YCSB batches without staging of up to
+                                 8,192 lanes a multiprocessor (1 op per thread,
+                                 32 / ops_per_txn transactions to 32 lanes), and
+                                 persistent ones, take one per key per block
+                                 whatever this says                             */
     uint32_t late_reads;      /* YCSB: rows read after the check (see above):
                                  1 = in the check kernel's tiles, 2 = in a kernel
                                  of their own, 3 = write-first registration

@@ -137,8 +137,8 @@ struct TxnCounts {
 // The four counters share one 32-byte sector, whose reductions retire one
 // after another (1.56 G/s measured): one set per warp kept the write-back of a
 // 2^20-transaction YCSB batch waiting (9,728 warps: 36 us, of which 25 were
-// these), so a block sends one set.  Its last warp does, as the first thread
-// goes on to finish_batch, whose fence would wait for reductions of its own.
+// these), so a block sends one set.  Its last warp does, while the first thread
+// goes on to finish_batch.
 __device__ __forceinline__ void add_counters(DevStats *st, DevCtl *ctl, const TxnCounts &c) {
     __shared__ uint32_t cnt[4][32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;

@@ -640,12 +640,11 @@ struct TpccTunedArgs {
     DevCtl *ctl;
     uint32_t filter;
     uint32_t dedupe;  // one registration per distinct slot of a warp (header ops)
-    // claims (see below): claimed rows' bits and rows claimed twice, claim_words
+    // claims (see below): claimed rows' bits and rows claimed twice, claim_words(W)
     // words each; whether there are any of the latter, and any StockLevel; the
     // STOCK rows that StockLevels read; the STOCK rows' smallest writers
     uint32_t *claim, *multi, *any, *sl_bits;
     unsigned long long *stock_w;
-    uint32_t claim_words;
 };
 enum : uint32_t { ANY_MULTI = 0, ANY_STOCKLEVEL = 1 };
 
@@ -1366,10 +1365,9 @@ cudaError_t tpcc_run_tuned(ltpg_ctx *c, Slot &s, int mode) {
     a.ctl = c->ctl;
     a.filter = c->launch_c.filter;
     a.dedupe = c->launch_c.dedupe;
-    a.claim_words = claim_words(a.db.W);
     a.claim = c->tpcc.claim;
-    a.multi = a.claim + a.claim_words;
-    a.any = a.multi + a.claim_words;
+    a.multi = a.claim + claim_words(a.db.W);
+    a.any = a.multi + claim_words(a.db.W);
     a.sl_bits = a.any + 2;
     a.stock_w = c->tpcc.stock_w;
     const bool claim = mode != LTPG_MODE_PERSISTENT && c->tpcc.claim && tpcc_claims(s, c->tpcc);

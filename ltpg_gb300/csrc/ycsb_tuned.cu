@@ -78,6 +78,10 @@ __device__ __forceinline__ uint32_t ld_ca_u32(const unsigned *p) {
 // return a line cached before the grid barrier.  Op words, values and rows
 // (read before the write-back) are written by no phase and keep the
 // read-only path.  In the separate kernels L1 starts empty at every kernel.
+// One exception: checkwb_tiles loads the slots through L1 in the persistent
+// kernel too.  No thread loads a slot between its block's arrival at the grid
+// barrier and the barrier's fence (thread 0's __threadfence behind the wait,
+// then __syncthreads), after which a load does not see what L1 held before.
 template <bool kCoh>
 __device__ __forceinline__ uint64_t ld_filter_u64(const unsigned long long *p) {
     return kCoh ? ld_gpu_u64(p) : ld_ca_u64(p);
@@ -407,7 +411,6 @@ __device__ __forceinline__ void wf_register_writes(const YcsbTunedArgs &a, uint6
 
 // One key of a read that has a writer: RAW against the final write word, and
 // the read's registration.  Returns the RAW bit.
-template <bool kCoh>
 __device__ __forceinline__ bool wf_read_key(const YcsbTunedArgs &a, uint32_t key, uint32_t t,
                                             uint32_t epoch, const ulonglong2 &s) {
     const unsigned long long mine = slot_tag(epoch) | t;
@@ -436,7 +439,7 @@ __device__ __forceinline__ bool wf_read_rest(const YcsbTunedArgs &a, uint32_t w,
     bool raw = false;
     for (; m; m &= m - 1u) {
         const uint32_t key = k1 + (uint32_t)__ffs(m) - 1u;
-        raw |= wf_read_key<kCoh>(a, key, t, epoch, ld_reg<kCoh>(a.reg + key));
+        raw |= wf_read_key(a, key, t, epoch, ld_reg<kCoh>(a.reg + key));
     }
     return raw;
 }
@@ -528,7 +531,7 @@ __device__ __forceinline__ void wf_register_reads(const YcsbTunedArgs &a, uint32
         bool raw = false;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            raw |= wf_read_key<kCoh>(a, ycsb_key(words[q]), t, epoch, s[q]);
+            raw |= wf_read_key(a, ycsb_key(words[q]), t, epoch, s[q]);
             if (rd[q] && ycsb_span(words[q])) raw |= wf_read_rest<kCoh>(a, words[q], t, epoch);
         }
         // one atomic per transaction: the lowest of its threads in the warp
@@ -1375,10 +1378,12 @@ static uint64_t lanes_of(const YcsbTunedArgs &a) { return 32ull * ((a.B + a.grp 
 
 // A batch of up to about eight waves of lanes.  In one, a block registers a key
 // once whatever is asked for (65,536 x 10: theta 0.99 29 -> 21 us, 0 and 0.6
-// within 1 us); beyond, the barrier per step costs more than it saves (2^18 x 10
-// at theta 0.6: 48 -> 53 us).  And the check's launch overlaps the execute
-// kernel (65,536 x 10: 29.5 -> 27 us a batch); beyond, its early blocks are in
-// the way (2^20 x 10: 240 -> 242 us; with staging 414 -> 427).
+// within 1 us; the launch setting dedupe has no say then, and up to two steps a
+// warp most lanes look at the slot with filter off too); beyond, the barrier per
+// step costs more than it saves (2^18 x 10 at theta 0.6: 48 -> 53 us).  And the
+// check's launch overlaps the execute kernel (65,536 x 10: 29.5 -> 27 us a
+// batch); beyond, its early blocks are in the way (2^20 x 10: 240 -> 242 us;
+// with staging 414 -> 427).
 static bool few_waves(const ltpg_ctx *c, const YcsbTunedArgs &a) {
     return lanes_of(a) <= 8192ull * c->sm_count;
 }
