@@ -935,7 +935,7 @@ def main():
         res, exact, e2e, batches = tpcc_bench(args, w, dist)
     rec = workload_record(args, w, theta, dist, res, exact, e2e, batches, peaks, peak_kind)
     # the TPC-C headline workload beside the YCSB one, with the YCSB run's
-    # access-pattern ceilings for its atomic roofline
+    # access-pattern ceilings
     tp = None
     if args.workload == "ycsb_hc" and not args.no_tpcc:
         wt = dict(WORKLOADS["tpcc"], key="tpcc")

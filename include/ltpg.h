@@ -552,7 +552,7 @@ typedef struct {
 int ltpg_server_open(ltpg_ctx *tpcc_ctx, ltpg_ctx *ycsb_ctx, const ltpg_server_cfg *cfg, ltpg_server **out);
 /* Admits n requests (copied before return); their ids are *first_id .. + n-1.
  * A request's submit time, from which its waiting and latency count, is when
- * the call reached it, to within 32 requests. */
+ * the call reached it, to within 128 requests. */
 int ltpg_serve_submit(ltpg_server *s, const ltpg_request *reqs, uint32_t n, uint64_t *first_id);
 /* Results of requests first_id .. first_id + n - 1: *n_done = how many of them,
  * from first_id on, have finished; their flags (LTPG_FLAG_*) and results are

@@ -351,10 +351,12 @@ int submit(ltpg_server *s, const ltpg_request *reqs, uint32_t n, uint64_t *first
     int r = progress(s);
     if (r) return r;
     if (first_id) *first_id = s->next_id;
-    double now = 0;  // looked at every 32 requests and after every wait: a look takes 32 ns, packing a request 23
+    // Looked at every 128 requests (3 us of packing: a look takes 32 ns, packing a
+    // request 23) and after every wait; every 32 cost a 2,000-request pass 2 us.
+    double now = 0;
     for (uint32_t i = 0; i < n; ++i) {
         const ltpg_request &q = reqs[i];
-        if (!t_submit && i % 32u == 0u) now = s->now();
+        if (!t_submit && i % 128u == 0u) now = s->now();
         if ((r = check_request(s, q))) return r;
         const double t = t_submit ? t_submit[i] : now;
         const bool lines_full =
