@@ -1066,35 +1066,61 @@ __device__ __forceinline__ void coop_exec_loop(const YcsbTunedArgs &a, StageEnt 
             const bool rd = act && !ycsb_is_pad(w) && ycsb_key(w) < a.n && ycsb_span(w) != 0u;
             const uint32_t key = ycsb_key(w);
             const uint32_t last = rd ? (uint32_t)scan_last(w, a.n) : 0u;
-            // the warp takes its scans one at a time: all lanes read the
-            // scan's rows as one contiguous range (16 B chunks, coalesced) and
-            // register its keys after the first, one key per lane
+            // eight lanes to a scan, four scans of the warp at a time: its rows
+            // by the 128-byte lines they cover, two lines in flight, and its
+            // keys after the first, one per lane
             unsigned long long xf = 0, xa = 0;  // this lane's scan: first row, all rows
-            for (unsigned m = __ballot_sync(FULL, rd); m; m &= m - 1u) {
-                const uint32_t src = (uint32_t)__ffs(m) - 1u;
-                const uint32_t k0 = __shfl_sync(FULL, key, src), k1 = __shfl_sync(FULL, last, src);
-                const uint32_t ts = __shfl_sync(FULL, t, src);
-                const uint32_t chunks = kReads ? (k1 - k0 + 1u) * 5u : 0u;
-                const ulonglong2 *p = reinterpret_cast<const ulonglong2 *>(a.rows + (uint64_t)k0 * LTPG_YCSB_FIELDS);
-                unsigned long long c_all = 0, c_first = 0;
-                for (uint32_t c = lane; c < chunks; c += 32u) {
-                    const ulonglong2 q = ld_nc16(p + c);
-                    c_all ^= q.x ^ q.y;
-                    if (c < 5u) c_first ^= q.x ^ q.y;
+            for (unsigned m = __ballot_sync(FULL, rd); m;) {
+                uint32_t own[4], src = lane;
+                bool have = false;
+#pragma unroll
+                for (uint32_t g = 0; g < 4; ++g) {
+                    own[g] = m ? (uint32_t)__ffs(m) - 1u : 32u;
+                    if (lane >> 3 == g && m) {
+                        src = own[g];
+                        have = true;
+                    }
+                    m &= m - 1u;
                 }
-                if (lane < k1 - k0) {
-                    unsigned long long *slot = &a.reg[(uint64_t)k0 + 1u + lane].r;
-                    const unsigned long long mine = tag | ts;
+                const uint32_t k0 = __shfl_sync(FULL, key, src), rest = __shfl_sync(FULL, last - key, src);
+                const unsigned long long mine = tag | __shfl_sync(FULL, t, src);
+                const uint32_t l = lane & 7u;
+                unsigned long long c_all = 0, c_first = 0;
+                if (kReads && have) {
+                    const uint64_t first = (uint64_t)k0 * 5u;  // in chunks of the table
+                    const uint32_t off = (uint32_t)first & 7u, end = off + (rest + 1u) * 5u;
+                    const ulonglong2 *p = reinterpret_cast<const ulonglong2 *>(a.rows) + (first - off);
+                    for (uint32_t q = l; q < end; q += 16u) {
+                        ulonglong2 v[2];
+#pragma unroll
+                        for (uint32_t r = 0; r < 2; ++r) {
+                            const uint32_t at = q + 8u * r;
+                            v[r] = at >= off && at < end ? ld_nc16_issue(p + at) : make_ulonglong2(0ull, 0ull);
+                        }
+#pragma unroll
+                        for (uint32_t r = 0; r < 2; ++r) {
+                            c_all ^= v[r].x ^ v[r].y;
+                            if (q + 8u * r < off + 5u) c_first ^= v[r].x ^ v[r].y;
+                        }
+                    }
+                }
+                for (uint32_t i = l; have && i < rest; i += 8u) {
+                    unsigned long long *slot = &a.reg[(uint64_t)k0 + 1u + i].r;
                     if (!kFilter || ld_ca_u64(slot) > mine) red_min(slot, mine);
                 }
                 if (!kReads) continue;
-                for (uint32_t o = 16; o >= 1u; o >>= 1) {
+#pragma unroll
+                for (uint32_t o = 4; o >= 1u; o >>= 1) {
                     c_all ^= __shfl_xor_sync(FULL, c_all, o);
                     c_first ^= __shfl_xor_sync(FULL, c_first, o);
                 }
-                if (lane == src) {
-                    xa = c_all;
-                    xf = c_first;
+#pragma unroll
+                for (uint32_t g = 0; g < 4; ++g) {
+                    const unsigned long long ga = __shfl_sync(FULL, c_all, 8u * g), gf = __shfl_sync(FULL, c_first, 8u * g);
+                    if (lane == own[g]) {
+                        xa = ga;
+                        xf = gf;
+                    }
                 }
             }
             if (!kReads) continue;
