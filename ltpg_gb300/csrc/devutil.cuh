@@ -114,12 +114,25 @@ __device__ __forceinline__ unsigned long long scan_rest(RegSlot *reg, const uint
     }
     return x;
 }
-// RAW on the keys of a range-scan read after its first.
+// Write word of a slot, nobody's when off.
+__device__ __forceinline__ uint64_t ld_writer_if(bool on, const RegSlot *p) {
+    uint64_t v = ~0ull;
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %2, 0; @q ld.global.cg.u64 %0, [%1]; }"
+                 : "+l"(v) : "l"(&p->w), "r"((uint32_t)on));
+    return v;
+}
+// RAW on the keys of a range-scan read after its first, four looks in flight.
 __device__ __forceinline__ bool scan_rest_raw(const RegSlot *reg, uint64_t n, uint32_t w, uint32_t t, uint32_t epoch) {
     if (!ycsb_span(w)) return false;
     const uint64_t last = scan_last(w, n);
     bool raw = false;
-    for (uint64_t q = (uint64_t)ycsb_key(w) + 1; q <= last; ++q) raw |= slot_min(ld_slot(reg + q).y, epoch) < t;
+    for (uint64_t q = (uint64_t)ycsb_key(w) + 1; q <= last; q += 4) {
+        uint64_t v[4];
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) v[i] = ld_writer_if(q + i <= last, reg + q + i);
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) raw |= slot_min(v[i], epoch) < t;
+    }
     return raw;
 }
 

@@ -669,7 +669,7 @@ __device__ __forceinline__ void checkwb_tiles(const YcsbTunedArgs &a, const Smem
             const uint32_t lt = v / vpt, t = t0 + lt;
             if (v >= blockDim.x) w4 = ld_nc_u4(vp + v);
             const uint32_t words[4] = {w4.x, w4.y, w4.z, w4.w};
-            uint32_t f = 0;
+            uint32_t f = 0, scans = 0;
             ulonglong2 s[2];  // two slots in flight: four take the registers of a block
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -683,9 +683,17 @@ __device__ __forceinline__ void checkwb_tiles(const YcsbTunedArgs &a, const Smem
                 if (ycsb_is_update(w)) {
                     if (rmin < t) f |= LTPG_FLAG_WAR;
                     if (wmin < t) f |= LTPG_FLAG_WAW;
-                } else if (wmin < t || (!ycsb_is_pad(w) && ycsb_key(w) < a.n && scan_rest_raw(a.reg, a.n, w, t, epoch))) {
-                    f |= LTPG_FLAG_RAW;
+                } else {
+                    if (wmin < t) f |= LTPG_FLAG_RAW;
+                    scans |= ycsb_span(w) != 0u && !ycsb_is_pad(w) && ycsb_key(w) < a.n ? 1u << q : 0u;
                 }
+            }
+            // range scans' other keys, out of the loop above: inside it they left
+            // one slot load in flight
+            for (; scans && !(f & LTPG_FLAG_RAW); scans &= scans - 1u) {
+                const uint32_t q = (uint32_t)__ffs(scans) - 1u;
+                const uint32_t w = q & 2u ? (q & 1u ? w4.w : w4.z) : q & 1u ? w4.y : w4.x;
+                if (scan_rest_raw(a.reg, a.n, w, t, epoch)) f |= LTPG_FLAG_RAW;
             }
             if (f) atomicOr(&fl[lt], f);
             if (!kLate) sm.upd[v] = (uint8_t)vec_updates(words);
