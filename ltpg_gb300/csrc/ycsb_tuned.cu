@@ -1166,6 +1166,105 @@ __global__ void __launch_bounds__(BS) ycsb_exec_coop(YcsbTunedArgs a) {
     }
 }
 
+// ---- execute + register by block tiles (ops_per_thread = 8) --------------------
+// Four op words per thread in one load, the rows one thread each, the registrations
+// through a warp dedupe; a tile's digests in shared memory.  Staging and batches
+// beyond a few waves take it when 8 is asked for: there it beats the cooperative
+// kernel on short scans and on staged updates (us for two batches: 488,324 x 3
+// scans of 2 keys 326 against 448, 112,203 x 8 staged updates 130 against 191);
+// on batches of a few waves the cooperative kernel is the faster one.
+template <bool kStage>
+__device__ __forceinline__ void exec_tiles(const YcsbTunedArgs &a, unsigned long long *dig, StageEnt *tab,
+                                           uint64_t tag) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t nvec_tile = a.tile * a.stride / 4;
+    const uint32_t n_tiles = (a.B + a.tile - 1) / a.tile;
+    for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+        const uint32_t t0 = tile * a.tile;
+        const uint32_t nt = min(a.tile, a.B - t0);
+        const uint32_t nvec = nt * a.stride / 4;
+        for (uint32_t i = threadIdx.x; i < a.tile; i += blockDim.x) dig[i] = 0ull;
+        __syncthreads();
+        const uint4 *vp = reinterpret_cast<const uint4 *>(a.ops + (uint64_t)t0 * a.stride);
+        for (uint32_t base = 0; base < nvec_tile; base += blockDim.x) {
+            const uint32_t v = base + threadIdx.x;
+            const bool act = v < nvec;
+            const uint4 w4 = act ? ld_nc_u4(vp + v) : make_uint4(LTPG_YCSB_OP_PAD, LTPG_YCSB_OP_PAD,
+                                                                  LTPG_YCSB_OP_PAD, LTPG_YCSB_OP_PAD);
+            const uint32_t lt = act ? (v * 4) / a.stride : 0;
+            const uint32_t j0 = v * 4 - lt * a.stride;
+            const uint32_t t = t0 + lt;
+            const uint32_t words[4] = {w4.x, w4.y, w4.z, w4.w};
+            unsigned long long part = 0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t w = words[q];
+                bool valid = act && !ycsb_is_pad(w);
+                const uint32_t key = ycsb_key(w);
+                const bool upd = ycsb_is_update(w);
+                if (valid && key >= a.n) {
+                    report_error(a.ctl, DERR_BOUNDS, t);
+                    valid = false;
+                }
+                bool staged = false;
+                if (kStage && valid) {
+                    const uint32_t b = key_bucket(key);
+                    const uint32_t g = __ldg(a.stage_map + b);
+                    if (g != STAGE_NONE && (g + 1) * a.ways <= a.stage_entries) {
+                        StageEnt *e = stage_find(tab, g, a.ways, key);
+                        if (e) {
+                            atomicMin(upd ? &e->wmin : &e->rmin, t);
+                            atomicAdd(&e->cnt, 1u);
+                            staged = true;
+                        }
+                    }
+                    if (!staged && (t % COUNT_SAMPLE) == 0u) atomicAdd(a.bucket_counts + b, COUNT_SAMPLE);
+                }
+                const bool need = valid && !staged;
+                const uint32_t mkey = need ? (key | (upd ? 0x80000000u : 0u)) : 0xFFFFFFFFu;
+                const unsigned peers = __match_any_sync(FULL, mkey);
+                // lanes are in transaction order, so the lowest peer holds the smallest TID
+                if (need && (__ffs(peers) - 1) == (int)lane) {
+                    unsigned long long *slot = upd ? &a.reg[key].w : &a.reg[key].r;
+                    const unsigned long long mine = tag | t;
+                    if (!a.filter || ld_ca_u64(slot) > mine) red_min(slot, mine);
+                }
+                if (valid && !upd) {
+                    const char *p = reinterpret_cast<const char *>(a.rows + (uint64_t)key * LTPG_YCSB_FIELDS);
+                    const ulonglong2 r0 = ld_nc16(p), r1 = ld_nc16(p + 16), r2 = ld_nc16(p + 32),
+                                     r3 = ld_nc16(p + 48), r4 = ld_nc16(p + 64);
+                    const unsigned long long x = r0.x ^ r0.y ^ r1.x ^ r1.y ^ r2.x ^ r2.y ^ r3.x ^ r3.y ^ r4.x ^ r4.y ^
+                                                 scan_rest(a.reg, a.rows, a.n, w, tag | t, a.filter != 0u);
+                    part += x * (2ull * (j0 + q) + 1ull);
+                }
+            }
+            if (part) atomicAdd(&dig[lt], part);
+        }
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < nt; i += blockDim.x) a.results[t0 + i] = (int64_t)dig[i];
+    }
+}
+
+// Shared memory: [dig: tile u64][stage table]; a tile is a multiple of 32.
+template <bool kStage>
+__global__ void __launch_bounds__(512) ycsb_exec_tiles(YcsbTunedArgs a) {
+    extern __shared__ __align__(16) char smem[];
+    unsigned long long *dig = reinterpret_cast<unsigned long long *>(smem);
+    StageEnt *tab = reinterpret_cast<StageEnt *>(dig + a.tile);
+    const uint64_t tag = slot_tag(a.ctl->epoch);
+    if (!kStage) clear_stats(a.st);
+    if (kStage) {
+        stage_init(tab, a.stage_entries);
+        __syncthreads();
+    }
+    exec_tiles<kStage>(a, dig, tab, tag);
+    if (kStage) {
+        __syncthreads();
+        const uint32_t ops = stage_flush(tab, a.stage_entries, a.reg, tag, a.bucket_counts);
+        if (ops) red_add_u64(&a.st->staged_ops, ops);
+    }
+}
+
 // Registers for three blocks of 512 an SM (two when rows are gathered here).
 template <int kLate>
 __global__ void __launch_bounds__(512, kLate == 1 ? 2 : 3) ycsb_checkwb_tuned(YcsbTunedArgs a) {
@@ -1504,12 +1603,32 @@ static cudaError_t launch_write_first(ltpg_ctx *c, const YcsbTunedArgs &a) {
     return with_block(c->launch_y.block, [&](auto bs) { return launch_write_first_t<decltype(bs)::value>(c, a); });
 }
 
+static void launch_tiles(ltpg_ctx *c, const YcsbTunedArgs &a, uint32_t tile, bool stage) {
+    const LaunchCfg &L = c->launch_y;
+    YcsbTunedArgs t = a;
+    t.tile = tile;
+    const size_t smem = (size_t)tile * 8 + (stage ? (size_t)a.stage_entries * sizeof(StageEnt) : 0);
+    void (*k)(YcsbTunedArgs) = stage ? ycsb_exec_tiles<true> : ycsb_exec_tiles<false>;
+    if (smem + static_smem((const void *)k) > 48 * 1024)
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, (int)L.block, smem);
+    if (per_sm < 1) per_sm = 1;
+    if (L.blocks_per_sm && (int)L.blocks_per_sm < per_sm) per_sm = (int)L.blocks_per_sm;
+    k<<<std::min((a.B + tile - 1) / tile, (uint32_t)(per_sm * c->sm_count)), L.block, smem, c->stream>>>(t);
+}
+
 // Launch shapes of the execute phase, by ops_per_thread: 2 / 4 = per-thread row
-// reads (ycsb_exec_fast) where stride / ops is a power of two, otherwise
-// cooperative row reads (ycsb_exec_coop).
-static void launch_exec(ltpg_ctx *c, const YcsbTunedArgs &a, bool stage) {
+// reads (ycsb_exec_fast) where stride / ops is a power of two; 8 = block tiles of
+// `tile` transactions (ycsb_exec_tiles) with staging and beyond a few waves;
+// otherwise cooperative row reads (ycsb_exec_coop).
+static void launch_exec(ltpg_ctx *c, const YcsbTunedArgs &a, uint32_t tile, bool stage) {
     const uint32_t ops = c->launch_y.per_thread ? c->launch_y.per_thread : 4u;
     const uint32_t lpt = a.stride / ops;
+    if (ops == 8u && (stage || !few_waves(c, a))) {
+        launch_tiles(c, a, tile, stage);
+        return;
+    }
     if ((ops != 2u && ops != 4u) || (lpt & (lpt - 1))) {
         launch_coop(c, a, stage, true);
         return;
@@ -1592,6 +1711,7 @@ cudaError_t ycsb_run_tuned(ltpg_ctx *c, Slot &s, int mode) {
     // A batch of less than one wave is spread over all resident blocks: the
     // kernels are chains of dependent accesses, which more threads shorten.
     const uint32_t resident = (uint32_t)(per_sm * c->sm_count);
+    const uint32_t full_tile = a.tile;
     a.tile = std::min(a.tile, ((a.B + resident - 1) / resident + 31u) / 32u * 32u);
     const uint32_t n_tiles = (a.B + a.tile - 1) / a.tile;
     if (persistent) {
@@ -1610,7 +1730,7 @@ cudaError_t ycsb_run_tuned(ltpg_ctx *c, Slot &s, int mode) {
     prof_mark(c, 0);
     count_launch(c);
     if (late) launch_coop(c, a, stage, false);
-    else launch_exec(c, a, stage);
+    else launch_exec(c, a, full_tile, stage);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     prof_mark(c, 1);
     count_launch(c);

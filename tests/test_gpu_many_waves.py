@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 import oracle
-from ltpg_gb300 import Engine, YcsbGenerator, abi
+from ltpg_gb300 import Engine, YcsbGenerator, abi, key_bucket
 
 pytestmark = pytest.mark.gpu
 
@@ -64,5 +64,34 @@ def test_scans(gpu, k):
             assert np.array_equal(e.txn_flags(0, B), want[0])
             assert np.array_equal(e.txn_results(0, B), want[2])
             assert np.array_equal(e.download_table(abi.TABLE_YCSB), o.rows)
+    finally:
+        e.close()
+
+
+@pytest.mark.parametrize("staged", [False, True])
+@pytest.mark.parametrize("threads", [128, 512])
+@pytest.mark.parametrize("k,scan", [(1, 0), (3, 2), (10, 0), (16, 5), (32, 0)])
+def test_tiles(gpu, k, scan, threads, staged):
+    """Eight ops per thread: block tiles, past the threshold or with staging."""
+    n = 50_000
+    B = 5001 if staged else _past_the_threshold(k)
+    b = YcsbGenerator(7, n, B, k, 30, 0.99, 0, scan).batch(0)
+    o = oracle.YcsbOracle(7, n)
+    want = o.run(b)
+    e = Engine(device=0, n_slots=1, max_txn=B, max_ops_per_txn=k)
+    try:
+        for filt in (0, 1):
+            e.load_ycsb(7, n)
+            e.set_launch("ycsb", block_threads=threads, ops_per_thread=8, filter=filt, dedupe=0, late_reads=0)
+            if staged:
+                e.stage_set(key_bucket(np.arange(100)))
+            e.upload(0, b)
+            e.run_batch(0, "graph" if filt else "fused")
+            e.sync()
+            assert np.array_equal(e.txn_flags(0, B), want[0])
+            assert np.array_equal(e.commit_bitmap(0, B), want[1])
+            assert np.array_equal(e.txn_results(0, B), want[2])
+            assert np.array_equal(e.download_table(abi.TABLE_YCSB), o.rows)
+            assert (e.stats(0)["staged_ops"] > 0) == staged
     finally:
         e.close()
