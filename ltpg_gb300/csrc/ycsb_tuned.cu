@@ -1715,8 +1715,14 @@ cudaError_t ycsb_run_tuned(ltpg_ctx *c, Slot &s, int mode) {
     a.tile = std::min(a.tile, ((a.B + resident - 1) / resident + 31u) / 32u * 32u);
     const uint32_t n_tiles = (a.B + a.tile - 1) / a.tile;
     if (persistent) {
-        // a lane per op in the first phase
-        const uint64_t blocks = std::max<uint64_t>(n_tiles, (lanes_of(a) + threads - 1) / threads);
+        // A lane per op in the first phase.  The write-first phases take a block to
+        // a full tile where that fills half of the multiprocessors: more blocks only send
+        // more of the hot keys' registrations at once (us for two batches, filter
+        // off, theta 0.999: 30,273 x 16 285 with all resident blocks, 230 so;
+        // 58,782 x 3 168 and 121; 158 x 32, which does not fill them, 59 and 84).
+        const uint32_t full = (a.B + full_tile - 1) / full_tile;
+        const bool tiles = late_mode == 3u && full >= (uint32_t)c->sm_count / 2u;
+        const uint64_t blocks = tiles ? full : std::max<uint64_t>(n_tiles, (lanes_of(a) + threads - 1) / threads);
         const uint32_t grid = (uint32_t)std::min<uint64_t>(resident, blocks);
         prof_mark(c, 0);
         void *args[] = {&a};
