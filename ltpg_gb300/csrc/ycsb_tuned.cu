@@ -367,6 +367,7 @@ __device__ __forceinline__ ulonglong2 ld_slot_ca(const RegSlot *p) {
     return v;
 }
 
+constexpr uint32_t WF_FEW = 16;  // of a warp's 128 ops
 // (1) the updates' registrations and writer bits: four op words per thread
 // (transactions are 4-word aligned); every op's key is bounds-checked here.
 // Also zeroes the flag bytes, which (2) and (3) OR the conflict bits into.
@@ -378,32 +379,60 @@ __device__ __forceinline__ void wf_register_writes(const YcsbTunedArgs &a, uint6
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (a.B + 3u) / 4u; i += step)
         reinterpret_cast<unsigned *>(a.flags)[i] = 0u;
     const uint4 *vp = reinterpret_cast<const uint4 *>(a.ops);
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nvec; v += step) {
-        const uint4 w4 = ld_nc_u4(vp + v);
+    // a block-uniform loop, so that whole warps reach the warp-wide sum below
+    for (uint32_t base = blockIdx.x * blockDim.x; base < nvec; base += step) {
+        const uint32_t v = base + threadIdx.x;
+        const uint4 w4 = v < nvec ? ld_nc_u4(vp + v)
+                                  : make_uint4(LTPG_YCSB_OP_PAD, LTPG_YCSB_OP_PAD, LTPG_YCSB_OP_PAD, LTPG_YCSB_OP_PAD);
         const uint32_t t = v / vpt;
         const uint32_t words[4] = {w4.x, w4.y, w4.z, w4.w};
-        // one op after another: a look that comes after the sends before it finds
-        // the hot keys registered.  With the looks of a vector in flight together
-        // every update of a hot key was sent and queued at its slot (65,536 x 16
-        // at theta 0.99, half updates: registration 74 -> 138 us)
+        const unsigned long long mine = tag | t;
+        bool upd[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const uint32_t w = words[q];
-            if (ycsb_is_pad(w)) continue;
-            const uint32_t key = ycsb_key(w);
-            if (key >= a.n) {
-                report_error(a.ctl, DERR_BOUNDS, t);
-                continue;
+            upd[q] = !ycsb_is_pad(w) && ycsb_is_update(w) && ycsb_key(w) < a.n;
+            if (!ycsb_is_pad(w) && ycsb_key(w) >= a.n) report_error(a.ctl, DERR_BOUNDS, t);
+        }
+        auto slot_of = [&](int q) { return &a.reg[ycsb_key(words[q])].w; };
+        auto look_slot = [&](int q) { return upd[q] && a.filter ? ld_filter_u64<kCoh>(slot_of(q)) : ~0ull; };
+        auto look_bit = [&](int q) {
+            unsigned *bw = a.wbits + (ycsb_key(words[q]) >> 5);
+            return !upd[q] ? ~0u : kCoh ? ld_gpu_u32(bw) : ld_ca_u32(bw);
+        };
+        // bits are only set within a batch: a bit seen set needs no atomic
+        // (hot keys' updates would otherwise all hit one word)
+        auto set_bit = [&](int q, uint32_t seen) {
+            const uint32_t key = ycsb_key(words[q]);
+            if (!((seen >> (key & 31u)) & 1u)) atomicOr(a.wbits + (key >> 5), 1u << (key & 31u));
+        };
+        // Few updates in the warp: the looks of a vector are in flight together, as
+        // one after another they were this pass (2^20 x 16, 5 % updates: 36 -> 27
+        // us; 50 -> 34 at theta 0).  Many: one op after another, as a look that
+        // comes after the sends before it finds the hot keys registered; together
+        // every update of a hot key was sent and queued at its slot (65,536 x 16 at
+        // theta 0.99, two batches, half updates: 163 us together, 78 so; all
+        // updates 288 and 134).
+        if (__reduce_add_sync(FULL, (uint32_t)upd[0] + upd[1] + upd[2] + upd[3]) <= WF_FEW) {
+            uint64_t cur[4];
+            uint32_t seen[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                cur[q] = look_slot(q);
+                seen[q] = look_bit(q);
             }
-            if (!ycsb_is_update(w)) continue;
-            unsigned long long *slot = &a.reg[key].w;
-            const unsigned long long mine = tag | t;
-            if (!a.filter || ld_filter_u64<kCoh>(slot) > mine) red_min(slot, mine);
-            // bits are only set within a batch: a bit seen set needs no atomic
-            // (hot keys' updates would otherwise all hit one word)
-            unsigned *bw = a.wbits + (key >> 5);
-            const uint32_t seen = kCoh ? ld_gpu_u32(bw) : ld_ca_u32(bw);
-            if (!((seen >> (key & 31u)) & 1u)) atomicOr(bw, 1u << (key & 31u));
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (upd[q] && cur[q] > mine) red_min(slot_of(q), mine);
+                set_bit(q, seen[q]);
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (!upd[q]) continue;
+                if (look_slot(q) > mine) red_min(slot_of(q), mine);
+                set_bit(q, look_bit(q));
+            }
         }
     }
 }
