@@ -166,6 +166,7 @@ struct YcsbGenArgs {
     uint32_t *ops, *val_off;
     uint64_t *vals;
     uint32_t tile;         // slots of a warp
+    bool perm_table;       // the permutation's rounds tabulated by each block
     uint32_t k_inv, s_inv; // ceil(2^16 / k), ceil(2^16 / stride): i / k = i k_inv >> 16 for a tile's indices
 };
 
@@ -221,7 +222,7 @@ __global__ void __launch_bounds__(GEN_T, 2) ycsb_gen_ops(YcsbGenArgs a) {
     __shared__ uint32_t next;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, k = a.p.ops_per_txn, stride = ycsb_stride(k), B = a.p.n_txn;
     const uint32_t half = a.perm.half, mask = (1u << half) - 1u, span = a.p.scan_len >= 2u ? a.p.scan_len - 1u : 0u;
-    const bool tabulated = a.rotate && half <= PERM_HALF;
+    const bool tabulated = a.perm_table;
     if (a.zipf.fast)
         for (uint32_t i = tid; i < POLY_CELLS * sizeof(PolyCell) / 16u; i += GEN_T)
             reinterpret_cast<uint4 *>(cells)[i] = reinterpret_cast<const uint4 *>(a.cells)[i];
@@ -337,6 +338,17 @@ __global__ void __launch_bounds__(GEN_T, 2) ycsb_gen_ops(YcsbGenArgs a) {
         }
         __syncwarp();
     }
+}
+
+// One thread per transaction: batches whose transactions repeat most of their
+// keys (each repeat draws the rest of the transaction again above), and the
+// smallest ones (gen_ycsb has the rule).
+__global__ void __launch_bounds__(TB) ycsb_gen_ops_txn(YcsbGenArgs a) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t == 0) a.val_off[0] = 0;
+    if (t >= a.p.n_txn) return;
+    a.val_off[t + 1] = ycsb_txn(a.p, a.zipf.z, *a.tab, a.rotate ? &a.perm : nullptr, a.batch_id, t,
+                                a.ops + (uint64_t)t * ycsb_stride(a.p.ops_per_txn));
 }
 
 // Update values, and the value offsets completed: val_off[t + 1] holds the
@@ -747,6 +759,7 @@ struct ltpg_gen_dev {
     FixTables *tab = nullptr;
     PolyCell *cells = nullptr;
     FastZipf zipf;
+    bool repeats = false;     // six redraws a transaction or more
     uint32_t gen_blocks = 0;  // resident blocks of ycsb_gen_ops on the device
     uint32_t G = 0, C = 0;
     uint32_t *o_id = nullptr, *no_id = nullptr, *ol_id = nullptr, *h_id = nullptr;
@@ -840,6 +853,22 @@ cudaError_t bind_tpcc(ltpg_gen *g, int device) {
     return cudaSuccess;
 }
 
+// Whether a transaction of k distinct ranks takes six redraws or more, from 32 of them.
+bool many_redraws(const Zipf &z, uint32_t k) {
+    Rng r(1);
+    uint32_t redraws = 0;
+    for (uint32_t t = 0; t < 32; ++t) {
+        uint64_t keys[LTPG_YCSB_MAX_OPS];
+        for (uint32_t j = 0; j < k; ++j)
+            for (uint32_t attempt = 0; attempt < 64; ++attempt) {
+                keys[j] = z.sample(r, host_fix_tables());
+                if (std::find(keys, keys + j, keys[j]) == keys + j) break;
+                if (++redraws >= 6 * 32) return true;
+            }
+    }
+    return false;
+}
+
 // The YCSB generator's power tables on the device (first device batch).
 cudaError_t bind_ycsb(ltpg_gen *g, int device) {
     ltpg_gen_dev *d = new (std::nothrow) ltpg_gen_dev();
@@ -847,6 +876,7 @@ cudaError_t bind_ycsb(ltpg_gen *g, int device) {
     d->device = device;
     std::vector<PolyCell> cells(POLY_CELLS);
     d->zipf = fast_zipf(g->zipf, cells.data());
+    d->repeats = many_redraws(g->zipf, g->y.ops_per_txn);
     cudaError_t e = dalloc(d, &d->tab, 1);
     if (e == cudaSuccess) e = cudaMemcpy(d->tab, &host_fix_tables(), sizeof(FixTables), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = dput(d, &d->cells, cells);
@@ -905,9 +935,23 @@ int gen_ycsb(ltpg_ctx *c, ltpg_gen *g, uint64_t batch_id, uint32_t slot, cudaStr
     a.tile = std::min(std::min<uint32_t>(32, GEN_WORDS / stride), std::max<uint32_t>(2, blocks(p.n_txn, warps)));
     a.k_inv = (65536u + p.ops_per_txn - 1) / p.ops_per_txn;
     a.s_inv = (65536u + stride - 1) / stride;
-    const uint32_t perm_bytes = a.rotate && a.perm.half <= PERM_HALF ? (4u << a.perm.half) * sizeof(uint16_t) : 0u;
-    ycsb_gen_ops<<<std::min(blocks(blocks(p.n_txn, a.tile), GEN_T / 32), g->dev->gen_blocks), GEN_T, GEN_BYTES + perm_bytes,
-                   st>>>(a);
+    const uint32_t grid = std::min(blocks(blocks(p.n_txn, a.tile), GEN_T / 32), g->dev->gen_blocks);
+    // a table of 4 x 2^half rounds pays from as many draws a block as its side is long
+    a.perm_table = a.rotate && a.perm.half <= PERM_HALF &&
+                   (uint64_t)p.n_txn * p.ops_per_txn / grid >= (1u << a.perm.half);
+    // One thread per transaction where that is the faster one (us, threads against
+    // slots): cheap draws, i.e. uniform keys in rank order (440,861 x 10: 48 against
+    // 73; not in small batches, 8,029 x 32: 33 against 23); transactions that
+    // redraw most of their keys (292,566 x 32 of 302 keys at theta 0.999: 1,040
+    // against 5,900; not in small batches either); and one or two keys in a small
+    // batch (12 against 14).
+    const bool small = p.n_txn <= 8192u, uniform = p.theta == 0.0 && !a.rotate;
+    const bool threads = (uniform && !small) || (g->dev->repeats && (uniform || !small)) ||
+                         (p.n_txn <= 4096u && (p.ops_per_txn == 1u || (p.ops_per_txn == 2u && !a.rotate)));
+    if (threads)
+        ycsb_gen_ops_txn<<<blocks(p.n_txn, TB), TB, 0, st>>>(a);
+    else
+        ycsb_gen_ops<<<grid, GEN_T, GEN_BYTES + (a.perm_table ? (4u << a.perm.half) * sizeof(uint16_t) : 0u), st>>>(a);
     count_launch(c);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) {
