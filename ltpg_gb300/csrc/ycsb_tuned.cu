@@ -716,11 +716,16 @@ __device__ __forceinline__ void checkwb_tiles(const YcsbTunedArgs &a, const Smem
                     if (wmin < t) f |= LTPG_FLAG_WAW;
                 } else {
                     if (wmin < t) f |= LTPG_FLAG_RAW;
-                    scans |= ycsb_span(w) != 0u && !ycsb_is_pad(w) && ycsb_key(w) < a.n ? 1u << q : 0u;
+                    if (ycsb_span(w) && !ycsb_is_pad(w) && ycsb_key(w) < a.n) {
+                        if (kLate != 1) scans |= 1u << q;
+                        else if (!(f & LTPG_FLAG_RAW) && scan_rest_raw(a.reg, a.n, w, t, epoch)) f |= LTPG_FLAG_RAW;
+                    }
                 }
             }
             // range scans' other keys, out of the loop above: inside it they left
-            // one slot load in flight
+            // one slot load in flight at 40 registers.  Not with late reads 1, which
+            // has more and whose row reads lost some of theirs to it (60,942 x 32
+            // persistent 84 -> 88 us).
             for (; scans && !(f & LTPG_FLAG_RAW); scans &= scans - 1u) {
                 const uint32_t q = (uint32_t)__ffs(scans) - 1u;
                 const uint32_t w = q & 2u ? (q & 1u ? w4.w : w4.z) : q & 1u ? w4.y : w4.x;
