@@ -1759,10 +1759,20 @@ cudaError_t ycsb_run_tuned(ltpg_ctx *c, Slot &s, int mode) {
         // more of the hot keys' registrations at once (us for two batches, filter
         // off, theta 0.999: 30,273 x 16 285 with all resident blocks, 230 so;
         // 58,782 x 3 168 and 121; 158 x 32, which does not fill them, 59 and 84).
+        // The other late reads meet at two or three barriers, and neighbouring blocks
+        // share a multiprocessor (of 1,824 the first 17 sit on four), which then do
+        // the later phases of a batch with fewer tiles than blocks: at most two
+        // blocks to a tile, and four of 128 threads to a multiprocessor (twelve fit;
+        // 12,630 x 32 updates 109 us with all of them, 63 so; of 256 threads all:
+        // 132,766 x 3 77 us, with four 121).
         const uint32_t full = (a.B + full_tile - 1) / full_tile;
         const bool tiles = late_mode == 3u && full >= (uint32_t)c->sm_count / 2u;
         const uint64_t blocks = tiles ? full : std::max<uint64_t>(n_tiles, (lanes_of(a) + threads - 1) / threads);
-        const uint32_t grid = (uint32_t)std::min<uint64_t>(resident, blocks);
+        const uint32_t few = std::max<uint32_t>(2u * n_tiles, c->sm_count);
+        const uint32_t most = late_mode == 1u || late_mode == 2u
+                                  ? std::max(full, std::min(few, threads < 256u ? 4u * c->sm_count : resident))
+                                  : resident;
+        const uint32_t grid = (uint32_t)std::min<uint64_t>(std::min(most, resident), blocks);
         prof_mark(c, 0);
         void *args[] = {&a};
         count_launch(c);
