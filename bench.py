@@ -257,11 +257,16 @@ def profile_traffic(workload, kernel):
     return None
 
 
-def ycsb_exec_kernel_name(launch, stride):
-    """Name of the execute kernel the tuned path launches for this shape."""
-    opt = (launch or {}).get("ops_per_thread", 1)
-    if not (launch or {}).get("late_reads") and opt in (2, 4) and ((stride // opt) & (stride // opt - 1)) == 0:
-        return "ycsb_exec_fast"
+def ycsb_exec_kernel_name(launch, n_txn, k):
+    """Name of the execute kernel the tuned path launches for this shape (no staging)."""
+    opt, stride = (launch or {}).get("ops_per_thread", 1), (k + 3) & ~3
+    if not (launch or {}).get("late_reads"):
+        if opt in (2, 4) and ((stride // opt) & (stride // opt - 1)) == 0:
+            return "ycsb_exec_fast"
+        if opt == 8:
+            import torch
+            if -(-n_txn // (32 // k)) * 32 > 8192 * torch.cuda.get_device_properties(0).multi_processor_count:
+                return "ycsb_exec_tiles"
     return "ycsb_exec_coop"
 
 
@@ -848,7 +853,7 @@ def workload_record(args, w, theta, dist, res, exact, e2e, batches, peaks, peak_
     if w["kind"] == "ycsb":
         eb, cb, rb, wb = ycsb_bytes_per_txn(w["ops"], w["update_pct"] / 100, commit_rate,
                                             max(1, w.get("scan_len", 0)), late)
-        ek = ycsb_exec_kernel_name(launch, (w["ops"] + 3) & ~3)
+        ek = ycsb_exec_kernel_name(launch, w["n_txn"], w["ops"])
         ck = "ycsb_checkwb_tuned"
         wk = "ycsb_writeback_late"
         if late == 3:  # the registration interval is two kernels; the reads' dominates

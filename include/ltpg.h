@@ -407,7 +407,8 @@ typedef struct {
                                  many transactions)                             */
     uint32_t ops_per_thread;  /* YCSB op words per thread: 1, 2, 4 or 8 (2 and 4
                                  where op_stride / ops_per_thread is a power of
-                                 two; otherwise as 1)                           */
+                                 two; 8, block tiles, with staging or beyond the
+                                 few waves that dedupe names; otherwise as 1)   */
     uint32_t blocks_per_sm;   /* cap on resident blocks per SM, 0 = occupancy   */
     uint32_t stage_ways;      /* shared-memory staging entries per hot bucket   */
     uint32_t filter;          /* 1 = read the slot before its atomicMin (where
